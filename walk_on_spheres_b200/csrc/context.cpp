@@ -279,6 +279,8 @@ void SceneDevice::set_views(const HostScene &h) {
     wide.box = static_cast<const float *>(at(4));
     wide.prim = static_cast<const float *>(at(5));
     wide.wide2bin = static_cast<const int *>(at(6));
+    const float m64 = fp32_distance_margin(h.bbox, h.dim);
+    wide.margin64 = wide64_usable(h.bbox, h.dim, m64) ? m64 : -1.0f;
     slot_verts = static_cast<const int *>(at(8));
 }
 
@@ -526,7 +528,7 @@ int wos_context::run(const wos_params &p, const PointSet &ps, Fields out,
              "classification kernel");
     WOS_CUDA(this, cudaEventRecord(events[1], stream), "event");
     if (p.method == WOS_METHOD_PLAIN_FP64) {
-        WOS_CUDA(this, launch_walk_plain(view, ps, p.seed, eq, p.N_walks, eps, p.max_steps, loc,
+        WOS_CUDA(this, launch_walk_plain(view, wide, ps, p.seed, eq, p.N_walks, eps, p.max_steps, loc,
                                          st, out, ctr, stream),
                  "plain walk kernel");
     } else {

@@ -6,6 +6,7 @@
 #include "prng.cuh"
 #include "scene.cuh"
 #include "wide.cuh"
+#include "wide64.cuh"
 
 namespace wosb {
 

@@ -77,6 +77,9 @@ struct WideView {
     // the primitive records again, one per wide slot, contiguous (2D: 5 of 8
     // floats, 3D: 16 floats), for the list scans' per-lane gathers
     const float4 *aos;
+    // FP32 bounds steer exact FP64 queries with this margin (wide64.cuh);
+    // negative: they may not (wide64_usable)
+    float margin64;
 };
 
 // Lattice value D at the node nearest to p and the distance r from p to it:

@@ -1,0 +1,194 @@
+// Warp-cooperative exact FP64 closest-point queries on the 32-wide tree.
+//
+// The per-thread FP64 query (nearest64) walks the binary tree alone: about 30
+// dependent node visits, and the 32 lanes of a warp take 32 different paths.
+// Here the whole warp answers one query: the FP32 boxes and slabs of the wide
+// tree only decide which leaf clusters can hold the nearest primitive, and
+// the primitives themselves are compared in FP64 with the reference's
+// expressions, so the winning distance is the minimum over all primitives and
+// has the same bits whichever tree found it.
+//
+// What makes the FP32 pruning safe: boxes and slabs are rounded outward when
+// they are built, and `margin` (a few tens of ulps of the largest coordinate)
+// covers the rounding of the point to FP32 and of the bound arithmetic.  A
+// cluster is skipped only when its bound exceeds the best distance found plus
+// twice that margin.  wide64_usable() says for which scenes the margin is
+// meaningful; others keep the per-thread query.
+#pragma once
+#include "scene.cuh"
+#include "wide.cuh"
+
+namespace wosb {
+
+// FP32 bounds of a scene with this box can steer FP64 queries: coordinates
+// whose squares stay normal FP32 numbers, and a margin small against the
+// scene (a box far from the origin would make every cluster a candidate).
+inline bool wide64_usable(const double bbox[6], int dim, float margin) {
+    double ext = 0.0, mag = 0.0;
+    for (int k = 0; k < dim; ++k) {
+        const double lo = bbox[2 * k], hi = bbox[2 * k + 1];
+        ext = ext > hi - lo ? ext : hi - lo;
+        mag = mag > (lo < 0 ? -lo : lo) ? mag : (lo < 0 ? -lo : lo);
+        mag = mag > (hi < 0 ? -hi : hi) ? mag : (hi < 0 ? -hi : hi);
+    }
+    return ext > 1e-9 && mag < 1e9 && static_cast<double>(margin) < 1e-3 * ext;
+}
+
+// Squared FP64 distance from p to the primitive in binary slot k and its
+// closest point (the leaf test of nearest64).
+template <int DIM>
+__device__ __forceinline__ double slot_dist64(const SceneView &s, int k, double px, double py,
+                                              double pz, double &nx, double &ny, double &nz) {
+    if (DIM == 2) {
+        const double2 a = s.seg64[2 * k], c = s.seg64[2 * k + 1];
+        nz = 0.0;
+        return npq_seg64(a.x, a.y, c.x, c.y, px, py, nx, ny);
+    }
+    const double2 *r = s.tri64 + 7 * k;
+    const double2 r0 = r[0], r1 = r[1], r2 = r[2], r3 = r[3], r4 = r[4], r5 = r[5], r6 = r[6];
+    return eberly<double>(px, py, pz, r0.x, r0.y, r1.x, r1.y, r2.x, r2.y, r3.x, r3.y, r4.x, r4.y,
+                          r5.x, r5.y, r6.x, r6.y, nx, ny, nz);
+}
+
+// Visits the leaf clusters whose FP32 lower bound is at most `limit` (which
+// leaf(cluster) lowers), nearest child first.  All 32 lanes call it with the
+// same point.
+template <int DIM, class Leaf>
+__device__ __forceinline__ void visit_clusters(const WideView &w, float px, float py, float pz,
+                                               const float &limit, Leaf &&leaf) {
+    constexpr unsigned kAll = 0xffffffffu;
+    const unsigned lane = threadIdx.x & 31u;
+    auto take_nearest = [&](unsigned &m, float d) -> int {
+        const unsigned key = ((m >> lane) & 1u) ? order_key(d, lane) : 0xffffffffu;
+        const unsigned k = __reduce_min_sync(kAll, key) & 31u;
+        m &= ~(1u << k);
+        return static_cast<int>(k);
+    };
+    if (w.H == 1) {
+        leaf(0);
+        return;
+    }
+    if (w.H == 2) {
+        const float d = wide_box_dist<DIM>(w, 1, 0, px, py, pz);
+        unsigned m = __ballot_sync(kAll, d <= limit);
+        while (m) {
+            leaf(take_nearest(m, d));
+            m &= __ballot_sync(kAll, d <= limit);
+        }
+        return;
+    }
+    // taller trees: above the two lowest levels, children in lane order with
+    // one pending mask per level; the two lowest nearest first
+    unsigned mask[8];
+    int parent[8];
+    int h = w.H - 1;
+    int node = 0;
+    float top = wide_box_dist<DIM>(w, h, 0, px, py, pz);
+    unsigned m2 = __ballot_sync(kAll, top <= limit);
+    for (;;) {
+        if (h == 2) {
+            while (m2) {
+                const int n2 = node * 32 + take_nearest(m2, top);
+                const float d1 = wide_box_dist<DIM>(w, 1, n2, px, py, pz);
+                unsigned m1 = __ballot_sync(kAll, d1 <= limit);
+                while (m1) {
+                    leaf(n2 * 32 + take_nearest(m1, d1));
+                    m1 &= __ballot_sync(kAll, d1 <= limit);
+                }
+                m2 &= __ballot_sync(kAll, top <= limit);
+            }
+        } else if (m2) {
+            const int child = node * 32 + take_nearest(m2, top);
+            mask[h] = m2;
+            parent[h] = node;
+            node = child;
+            --h;
+            top = wide_box_dist<DIM>(w, h, node, px, py, pz);
+            m2 = __ballot_sync(kAll, top <= limit);
+            continue;
+        }
+        // this node is done: back to its parent's pending children, whose
+        // bounds are formed again against the limit of now
+        if (h == w.H - 1) return;
+        ++h;
+        node = parent[h];
+        top = wide_box_dist<DIM>(w, h, node, px, py, pz);
+        m2 = mask[h] & __ballot_sync(kAll, top <= limit);
+    }
+}
+
+// The squared radius that still counts as a candidate once `best2` (a squared
+// FP32 distance, rounded up) has been found.
+__device__ __forceinline__ float candidate_limit(float best2, float margin) {
+    const float r = sqrtf(best2) + 2.0f * margin;
+    return r * r * (1.0f + 0x1p-20f);
+}
+
+// Lane minimum of non-negative doubles across the warp.
+__device__ __forceinline__ double warp_min_double(double v) {
+    const unsigned long long b = static_cast<unsigned long long>(__double_as_longlong(v));
+    const unsigned hi = static_cast<unsigned>(b >> 32), lo = static_cast<unsigned>(b);
+    const unsigned mh = __reduce_min_sync(0xffffffffu, hi);
+    const unsigned ml = __reduce_min_sync(0xffffffffu, hi == mh ? lo : 0xffffffffu);
+    return __longlong_as_double(static_cast<long long>(
+        (static_cast<unsigned long long>(mh) << 32) | ml));
+}
+
+// Binary slot of the primitive nearest to (px, py, pz), the same for all 32
+// lanes, which call it with the same point.  Equally near primitives: the
+// lowest slot, except that 2D primitives of different boundaries (a corner
+// where two boundaries meet) are decided by nearest64, so the boundary value
+// is the one the per-thread query picks.
+template <int DIM>
+__device__ __forceinline__ int warp_nearest64(const SceneView &s, const WideView &w, double px,
+                                              double py, double pz, float margin) {
+    constexpr unsigned kAll = 0xffffffffu;
+    const int lane = static_cast<int>(threadIdx.x & 31u);
+    const float fx = static_cast<float>(px), fy = static_cast<float>(py);
+    const float fz = static_cast<float>(pz);
+    // points outside the scene's box (classification) carry larger ulps
+    margin = fmaxf(margin, 4e-6f * fmaxf(fabsf(fx), fmaxf(fabsf(fy), fabsf(fz))));
+    double best = __longlong_as_double(0x7ff0000000000000LL);
+    int slot = -1;
+    bool split = false;  // this lane saw a tie across two boundaries
+    float limit = INFINITY, ubest = INFINITY;
+    visit_clusters<DIM>(w, fx, fy, fz, limit, [&](int cluster) {
+        const int ws = cluster * 32 + lane;
+        double d2 = __longlong_as_double(0x7ff0000000000000LL);
+        if (ws < w.n) {
+            const int k = __ldg(w.wide2bin + ws);
+            double nx, ny, nz;
+            d2 = slot_dist64<DIM>(s, k, px, py, pz, nx, ny, nz);
+            if (DIM == 2 && d2 == best && s.segid[k].x != s.segid[slot].x) split = true;
+            if (d2 < best || (d2 == best && k < slot)) {
+                if (d2 < best) split = false;
+                best = d2;
+                slot = k;
+            }
+        }
+        const float u = __uint_as_float(
+            __reduce_min_sync(kAll, __float_as_uint(__double2float_ru(d2))));
+        if (u < ubest) {
+            ubest = u;
+            limit = candidate_limit(u, margin);
+        }
+    });
+    const double m = warp_min_double(best);
+    const bool mine = best == m && slot >= 0;
+    const unsigned ties = __ballot_sync(kAll, mine);
+    if (!ties) return -1;
+    int win = __shfl_sync(kAll, slot, __ffs(ties) - 1);
+    if ((ties & (ties - 1u)) || __any_sync(kAll, mine && split)) {
+        win = static_cast<int>(
+            __reduce_min_sync(kAll, mine ? static_cast<unsigned>(slot) : 0xffffffffu));
+        if constexpr (DIM == 2) {
+            const int bid = s.segid[win].x;
+            if (__any_sync(kAll, mine && (split || s.segid[slot].x != bid))) {
+                win = nearest64<2>(s, px, py, pz, __longlong_as_double(0x7ff0000000000000LL)).slot;
+            }
+        }
+    }
+    return win;
+}
+
+}  // namespace wosb

@@ -51,8 +51,8 @@ cudaError_t launch_classify(const SceneView &s, const PointSet &ps, uint64_t see
 
 // PLAIN_FP64: every walk of every inside point on the point's reference
 // xoshiro256++ streams, in the reference order (include/wos/wos.hpp:54-191).
-cudaError_t launch_walk_plain(const SceneView &s, const PointSet &ps, uint64_t seed, EqDesc eq,
-                              int n_walks, double epsilon, int max_steps,
+cudaError_t launch_walk_plain(const SceneView &s, const WideView &w, const PointSet &ps,
+                              uint64_t seed, EqDesc eq, int n_walks, double epsilon, int max_steps,
                               const uint8_t *location, const StartRecord *start, Fields out,
                               DeviceCounters *counters, cudaStream_t stream);
 

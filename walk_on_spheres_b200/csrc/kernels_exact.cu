@@ -214,57 +214,76 @@ __global__ void __launch_bounds__(kExactThreads)
     }
 }
 
+// The walks of one point, one step of the current walk at a time.  A point's
+// walks run one after another on its streams (where a walk's draws begin
+// depends on every walk before it), so the point is the unit of parallel work.
 template <int DIM, class Eq>
-__global__ void __launch_bounds__(kExactThreads)
-    walk_plain_kernel(SceneView s, PointSet ps, uint64_t seed, Eq eq, int n_walks, double eps,
-                      int max_steps, const uint8_t *__restrict__ location,
-                      const StartRecord *__restrict__ start, Fields out, DeviceCounters *ctr) {
-    const long long stride = static_cast<long long>(gridDim.x) * blockDim.x;
-    for (long long t = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x; t < ps.n;
-         t += stride) {
-        if (location[t] != 1) continue;
-        double x, y, z;
+struct PlainWalks {
+    V3<double> x0, p, np;
+    double R0, R, sample, weight;
+    double mean, m2, total_steps;
+    unsigned long long steps_sum;
+    long long t;
+    int bid, i, steps, hits;
+    bool overflow;
+    Xoshiro walk, src;
+
+    __device__ PlainWalks(const PointSet &ps, long long point, uint64_t seed,
+                          const StartRecord *__restrict__ start)
+        : walk(0), src(0) {
+        t = point;
         uint64_t linear;
-        point_at(ps, t, x, y, z, linear);
+        point_at(ps, t, x0.x, x0.y, x0.z, linear);
         const uint64_t pseed = point_seed(seed, linear);
-        Xoshiro walk(splitmix64(pseed ^ kWalkStream));
-        Xoshiro src(DIM == 2 ? splitmix64(pseed ^ kSourceStream) : 0ull);
-        const StartRecord st = start[t];
-        double mean = 0.0, m2 = 0.0, total_steps = 0.0;
-        unsigned long long steps_sum = 0;
-        int hits = 0;
-        bool overflow = false;
-        for (int i = 0; i < n_walks; ++i) {
-            // wos_sample, include/wos/wos.hpp:54-138
-            V3<double> p{x, y, z};
-            V3<double> np{st.nx, st.ny, st.nz};
-            int bid = st.boundary_id;
-            double R = st.radius;
-            double sample = 0.0, weight = 1.0;
-            int steps = 0;
-            while (R > eps && steps < max_steps) {
-                if (DIM == 2) {
-                    p = walk_body<2, true, double>(eq, p, R, sample, weight, walk, src, overflow);
-                } else {
-                    p = walk_body<3, true, double>(eq, p, R, sample, weight, walk, walk, overflow);
-                }
-                ++steps;
-                const Nearest<double> q = nearest64<DIM>(s, p.x, p.y, p.z, dinf());
-                R = sqrt(q.best);
-                np = V3<double>{q.x, q.y, q.z};
-                if (DIM == 2) bid = s.segid[q.slot].x;
-            }
-            if (R > eps) ++hits;
-            sample += weight * eq.boundary(np, bid);
-            // Welford update, include/wos/wos.hpp:169-180
-            const double count = static_cast<double>(i + 1);
-            const double before = sample - mean;
-            mean += before / count;
-            const double after = sample - mean;
-            m2 += before * after;
-            total_steps += steps;
-            steps_sum += static_cast<unsigned long long>(steps);
+        walk = Xoshiro(splitmix64(pseed ^ kWalkStream));
+        src = Xoshiro(DIM == 2 ? splitmix64(pseed ^ kSourceStream) : 0ull);
+        R0 = start[t].radius;
+        mean = m2 = total_steps = 0.0;
+        steps_sum = 0;
+        i = hits = 0;
+        overflow = false;
+        begin();
+    }
+
+    // wos_sample, include/wos/wos.hpp:54-138
+    __device__ __forceinline__ void begin() {
+        p = x0;
+        R = R0;
+        sample = 0.0;
+        weight = 1.0;
+        steps = 0;
+    }
+    __device__ __forceinline__ bool stepping(double eps, int max_steps) const {
+        return R > eps && steps < max_steps;
+    }
+    __device__ __forceinline__ void step(const Eq &eq) {
+        if (DIM == 2) {
+            p = walk_body<2, true, double>(eq, p, R, sample, weight, walk, src, overflow);
+        } else {
+            p = walk_body<3, true, double>(eq, p, R, sample, weight, walk, walk, overflow);
         }
+        ++steps;
+    }
+    // The walk ends at its last nearest point (the start's, after no step).
+    __device__ __forceinline__ void end(const Eq &eq, double eps,
+                                        const StartRecord *__restrict__ start) {
+        if (steps == 0) {
+            np = V3<double>{start[t].nx, start[t].ny, start[t].nz};
+            bid = start[t].boundary_id;
+        }
+        if (R > eps) ++hits;
+        sample += weight * eq.boundary(np, bid);
+        // Welford update, include/wos/wos.hpp:169-180
+        const double count = static_cast<double>(i + 1);
+        const double before = sample - mean;
+        mean += before / count;
+        const double after = sample - mean;
+        m2 += before * after;
+        total_steps += steps;
+        steps_sum += static_cast<unsigned long long>(steps);
+        ++i;
+    }
+    __device__ void write(int n_walks, const Fields &out, DeviceCounters *ctr) const {
         const double variance = n_walks > 1 ? m2 / static_cast<double>(n_walks - 1) : 0.0;
         const double se = n_walks > 0 ? sqrt(variance / static_cast<double>(n_walks)) : 0.0;
         const double mean_steps = n_walks > 0 ? total_steps / static_cast<double>(n_walks) : 0.0;
@@ -277,6 +296,88 @@ __global__ void __launch_bounds__(kExactThreads)
         atomicAdd(&ctr->exact_queries, steps_sum);  // one FP64 BVH query per step
         atomicAdd(&ctr->total_walks, static_cast<unsigned long long>(n_walks));
         if (overflow) atomicOr(&ctr->error_flags, kErrRejectionCap);
+    }
+};
+
+// One thread per point, each with its own FP64 tree queries: the form for
+// scenes whose FP32 bounds cannot steer a query (wide64_usable).
+template <int DIM, class Eq>
+__global__ void __launch_bounds__(kExactThreads)
+    walk_plain_kernel(SceneView s, PointSet ps, uint64_t seed, Eq eq, int n_walks, double eps,
+                      int max_steps, const uint8_t *__restrict__ location,
+                      const StartRecord *__restrict__ start, Fields out, DeviceCounters *ctr) {
+    const long long stride = static_cast<long long>(gridDim.x) * blockDim.x;
+    for (long long t = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x; t < ps.n;
+         t += stride) {
+        if (location[t] != 1) continue;
+        PlainWalks<DIM, Eq> k(ps, t, seed, start);
+        while (k.i < n_walks) {
+            k.begin();
+            while (k.stepping(eps, max_steps)) {
+                k.step(eq);
+                const Nearest<double> q = nearest64<DIM>(s, k.p.x, k.p.y, k.p.z, dinf());
+                k.R = sqrt(q.best);
+                k.np = V3<double>{q.x, q.y, q.z};
+                if (DIM == 2) k.bid = s.segid[q.slot].x;
+            }
+            k.end(eq, eps, start);
+        }
+        k.write(n_walks, out, ctr);
+    }
+}
+
+// `per_warp` consecutive points per warp, one per lane; every iteration
+// steps each lane's walk and the whole warp then answers the lanes' queries
+// one after another (warp_nearest64).  A point's walks are serial, so the
+// kernel waits on one step's chain (draw, sine and cosine, query, square
+// root) rather than on issue slots.  Per-thread queries made that chain 30
+// dependent tree nodes long in 32 diverging lanes: 1360 inside points of an
+// annulus of 256 segments, 1000 walks, took 144.8 ms, now 11.9; 0.41 M walks
+// in a blob of 3968 triangles 425 ms, now 11.7 (same results, bit for bit).
+template <int DIM, class Eq>
+__global__ void __launch_bounds__(kExactThreads, 4)
+    walk_plain_warp_kernel(SceneView s, WideView w, int per_warp, PointSet ps, uint64_t seed,
+                           Eq eq, int n_walks, double eps, int max_steps,
+                           const uint8_t *__restrict__ location,
+                           const StartRecord *__restrict__ start, Fields out,
+                           DeviceCounters *ctr) {
+    constexpr unsigned kAll = 0xffffffffu;
+    __shared__ int s_off[8];
+    if (threadIdx.x < 8) s_off[threadIdx.x] = w.off[threadIdx.x];
+    __syncthreads();
+    w.off = s_off;
+    const int lane = threadIdx.x & 31;
+    const long long warp = (static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
+    const long long t = warp * per_warp + lane;
+    bool active = lane < per_warp && t < ps.n && location[t] == 1;
+    if (!__any_sync(kAll, active)) return;
+    PlainWalks<DIM, Eq> k(ps, active ? t : 0, seed, start);
+    while (__any_sync(kAll, active)) {
+        const bool query = active && k.stepping(eps, max_steps);
+        if (query) k.step(eq);
+        unsigned pending = __ballot_sync(kAll, query);
+        int slot = -1;
+        while (pending) {
+            const int j = __ffs(pending) - 1;
+            pending &= pending - 1u;
+            const double qx = __shfl_sync(kAll, k.p.x, j), qy = __shfl_sync(kAll, k.p.y, j);
+            const double qz = DIM == 3 ? __shfl_sync(kAll, k.p.z, j) : 0.0;
+            const int win = warp_nearest64<DIM>(s, w, qx, qy, qz, w.margin64);
+            if (lane == j) slot = win;
+        }
+        if (query) {
+            k.R = sqrt(slot_dist64<DIM>(s, slot, k.p.x, k.p.y, k.p.z, k.np.x, k.np.y, k.np.z));
+            if (DIM == 2) k.bid = s.segid[slot].x;
+        }
+        if (active && !k.stepping(eps, max_steps)) {
+            k.end(eq, eps, start);
+            if (k.i < n_walks) {
+                k.begin();
+            } else {
+                active = false;
+                k.write(n_walks, out, ctr);
+            }
+        }
     }
 }
 
@@ -313,47 +414,71 @@ int blocks_for(long long n, int threads) {
     return static_cast<int>(b);
 }
 
+// Points per warp of walk_plain_warp_kernel.  A warp answers its lanes'
+// queries in turn, so few points per warp give short steps, and many share
+// the cost of the step's arithmetic (one instruction stream for all lanes).
+// Measured on a B200, walk kernel in ms at 1 / 2 / 4 / 8 / 16 points per warp:
+// 2D circle of 1024 segments, 64 walks: 24^2 points 0.86 / 1.17 / 1.75 / 2.92
+// / 4.83; 64^2 1.50 / 1.28 / 1.94 / 3.14 / 5.36; 128^2 4.37 / 3.53 / 3.70 /
+// 3.57 / 5.66; 256^2 16.3 / 12.6 / 10.9 / 10.0 / 11.7.  3D sphere of 16 128
+// triangles, 16 walks (queries dominate the step): 24^3 3.88 / 4.15 / 4.37 /
+// 7.31 / 12.1; 40^3 15.4 / 14.4 / 14.7 / 16.5 / 18.3.
+int points_per_warp(int dim, long long n) {
+    if (dim == 3) return n >= 32768 ? 2 : 1;
+    int p = 1;
+    while (p < 8 && n / (2 * p) >= 2048) p *= 2;
+    return p;
+}
+
 template <int DIM, class Eq>
-void launch_plain_typed(const SceneView &s, const PointSet &ps, uint64_t seed, const Eq &eq,
+void launch_plain_typed(const SceneView &s, const WideView &w, const PointSet &ps, uint64_t seed, const Eq &eq,
                         int n_walks, double eps, int max_steps, const uint8_t *location,
                         const StartRecord *start, Fields out, DeviceCounters *ctr,
                         cudaStream_t stream) {
+    if (w.margin64 >= 0.0f) {
+        const int per_warp = points_per_warp(DIM, ps.n);
+        const long long warps = (ps.n + per_warp - 1) / per_warp;
+        walk_plain_warp_kernel<DIM, Eq>
+            <<<blocks_for(32 * warps, kExactThreads), kExactThreads, 0, stream>>>(
+                s, w, per_warp, ps, seed, eq, n_walks, eps, max_steps, location, start, out, ctr);
+        return;
+    }
     walk_plain_kernel<DIM, Eq><<<blocks_for(ps.n, kExactThreads), kExactThreads, 0, stream>>>(
         s, ps, seed, eq, n_walks, eps, max_steps, location, start, out, ctr);
 }
 
 template <int DIM>
-void launch_plain_dim(const SceneView &s, const PointSet &ps, uint64_t seed, EqDesc e,
+void launch_plain_dim(const SceneView &s, const WideView &w, const PointSet &ps, uint64_t seed, EqDesc e,
                       int n_walks, double eps, int max_steps, const uint8_t *location,
                       const StartRecord *start, Fields out, DeviceCounters *ctr,
                       cudaStream_t stream) {
     switch (e.kind) {
         case kLaplace:
-            launch_plain_typed<DIM>(s, ps, seed, Laplace<DIM>{}, n_walks, eps, max_steps,
+            launch_plain_typed<DIM>(s, w, ps, seed, Laplace<DIM>{}, n_walks, eps, max_steps,
                                     location, start, out, ctr, stream);
             break;
         case kPoisson:
-            launch_plain_typed<DIM>(s, ps, seed, Poisson<DIM>{e.mode, e.alpha}, n_walks, eps,
+            launch_plain_typed<DIM>(s, w, ps, seed, Poisson<DIM>{e.mode, e.alpha}, n_walks, eps,
                                     max_steps, location, start, out, ctr, stream);
             break;
         case kScreened:
-            launch_plain_typed<DIM>(s, ps, seed, Screened<DIM>{e.mode, e.alpha}, n_walks, eps,
+            launch_plain_typed<DIM>(s, w, ps, seed, Screened<DIM>{e.mode, e.alpha}, n_walks, eps,
                                     max_steps, location, start, out, ctr, stream);
             break;
         case kTransient:
             if (DIM == 2) {
-                launch_plain_typed<2>(s, ps, seed, Transient<2>{kGreen, e.alpha, e.tr}, n_walks,
+                launch_plain_typed<2>(s, w, ps, seed, Transient<2>{kGreen, e.alpha, e.tr}, n_walks,
                                       eps, max_steps, location, start, out, ctr, stream);
             }
             break;
         case kPlate:
             if (DIM == 2) {
-                launch_plain_typed<2>(s, ps, seed, Plate<2>{e.mode, *e.pl}, n_walks, eps,
+                launch_plain_typed<2>(s, w, ps, seed, Plate<2>{e.mode, *e.pl}, n_walks, eps,
                                       max_steps, location, start, out, ctr, stream);
             }
             break;
         default:
-            launch_plain_typed<DIM>(s, ps, seed, Helmholtz<DIM>{}, n_walks, eps, max_steps,
+            launch_plain_typed<DIM>(s, w, ps, seed, Helmholtz<DIM>{}, n_walks, eps, max_steps,
                                     location, start, out, ctr, stream);
             break;
     }
@@ -410,16 +535,16 @@ cudaError_t launch_classify_batch(int dim, const BatchItem *items, int n_items,
     return cudaGetLastError();
 }
 
-cudaError_t launch_walk_plain(const SceneView &s, const PointSet &ps, uint64_t seed, EqDesc eq,
-                              int n_walks, double eps, int max_steps, const uint8_t *location,
-                              const StartRecord *start, Fields out, DeviceCounters *counters,
-                              cudaStream_t stream) {
+cudaError_t launch_walk_plain(const SceneView &s, const WideView &w, const PointSet &ps,
+                              uint64_t seed, EqDesc eq, int n_walks, double eps, int max_steps,
+                              const uint8_t *location, const StartRecord *start, Fields out,
+                              DeviceCounters *counters, cudaStream_t stream) {
     if (ps.n <= 0) return cudaSuccess;
     if (s.dim == 2) {
-        launch_plain_dim<2>(s, ps, seed, eq, n_walks, eps, max_steps, location, start, out,
+        launch_plain_dim<2>(s, w, ps, seed, eq, n_walks, eps, max_steps, location, start, out,
                             counters, stream);
     } else {
-        launch_plain_dim<3>(s, ps, seed, eq, n_walks, eps, max_steps, location, start, out,
+        launch_plain_dim<3>(s, w, ps, seed, eq, n_walks, eps, max_steps, location, start, out,
                             counters, stream);
     }
     return cudaGetLastError();

@@ -142,7 +142,7 @@ extern "C" int wos_solve_grid_device_noalloc(wos_context *ctx, const wos_params 
     if (e != cudaSuccess) return fail(ctx, WOS_ERR_CUDA, std::string("classification kernel: ") + cudaGetErrorString(e));
     cudaEventRecord(ctx->events[1], s);
     if (!fast) {
-        e = wosb::launch_walk_plain(ctx->view, ps, p->seed, eq, p->N_walks, eps, p->max_steps, loc,
+        e = wosb::launch_walk_plain(ctx->view, ctx->wide, ps, p->seed, eq, p->N_walks, eps, p->max_steps, loc,
                                     start, out, ctr, s);
         cudaEventRecord(ctx->events[2], s);
     } else {

@@ -205,7 +205,7 @@ extern "C" int wos_stationary_solve(wos_context *ctx, const wos_stationary_param
     WOS_CUDA(ctx, cudaEventRecord(ctx->events[0], stream), "event");
     cudaError_t e = cudaSuccess;
     if (p.method == WOS_METHOD_PLAIN_FP64) {
-        e = launch_walk_plain(dev.view, ps, seed, eq, p.walks, p.epsilon, p.max_steps, loc, st,
+        e = launch_walk_plain(dev.view, dev.wide, ps, seed, eq, p.walks, p.epsilon, p.max_steps, loc, st,
                               out, ctr, stream);
     } else {
         const int precision = p.method == WOS_METHOD_FAST_FP64 ? 64 : 32;

@@ -301,7 +301,7 @@ extern "C" int wos_transient_solve(wos_context *ctx, const wos_transient_params 
                              se + static_cast<size_t>(s) * n, nullptr, nullptr};
             cudaError_t e2;
             if (p.method == WOS_METHOD_PLAIN_FP64) {
-                e2 = launch_walk_plain(dev.view, ps, seed, e, p.walks, p.epsilon, p.max_steps,
+                e2 = launch_walk_plain(dev.view, dev.wide, ps, seed, e, p.walks, p.epsilon, p.max_steps,
                                        loc, st, out, ctr + (s - 1), stream);
             } else {
                 e2 = launch_walk_fast(dev.view, dev.wide, ps, seed, e, p.walks, p.epsilon,
