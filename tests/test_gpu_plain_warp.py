@@ -71,3 +71,52 @@ def test_plain_walks_match_the_oracle(solver, oracle, name):
         assert np.all(np.abs(got - want)[~close] <= 4.0 * se[~close])
     steps = ref.mean_steps.reshape(loc.shape)[ins]
     assert np.array_equal(r.mean_steps[ins][close], steps[close])
+
+
+def _sliver_fan():
+    # a closed fan whose side triangles are up to 1e4 times longer than wide:
+    # their FP32 distances say little, so the queries must compare them in FP64
+    rng = np.random.default_rng(3)
+    n = 400
+    t = np.sort(rng.uniform(0.0, 2.0 * np.pi, n))
+    t[1::4] = t[::4] + 1e-4
+    ring = np.stack([np.cos(t), np.sin(t), np.zeros(n)], axis=1)
+    v = np.concatenate([ring, [[0.0, 0.0, 0.9], [0.0, 0.0, -0.9]]])
+    i = np.arange(n, dtype=np.int32)
+    j = np.roll(i, -1).astype(np.int32)
+    top = np.stack([i, j, np.full(n, n, np.int32)], axis=1)
+    bottom = np.stack([j, i, np.full(n, n + 1, np.int32)], axis=1)
+    p = np.concatenate([top, bottom]).astype(np.int32)
+    return Mesh(3, v, p, np.zeros(len(p), dtype=np.int32))
+
+
+@pytest.mark.parametrize("make", [_two_boundary_corner, _sliver_fan, lambda: _star(161),
+                                  lambda: meshes.uv_sphere(lon=40, lat=21)],
+                         ids=["corner", "slivers", "star161", "sphere"])
+def test_fp64_walks_take_exact_radii(solver, oracle, make):
+    """FAST_FP64 and PLAIN_FP64 with one step per walk: the walk ends at the
+    nearest boundary point of its first step, so a wrong nearest primitive
+    shows in the boundary value (PLAIN, point by point against the oracle) or
+    in the mean (FAST_FP64, within 4.5 standard errors at 99% of the points).
+    Where two boundaries meet in a corner, FAST_FP64 may take either one's
+    value (its distances round otherwise than the reference's, so equal ones
+    need not tie), and only PLAIN_FP64 is compared."""
+    from oracle.oracle import Solve
+    m = make()
+    solver.set_mesh(m)
+    n = (15, 13, 1) if m.dim == 2 else (9, 9, 9)
+    walks = 400
+    ref = oracle.solve_grid("laplace", Solve(m, *n, N_walks=walks, seed=5, max_steps=1))
+    r = solver.solve_grid("laplace", *n, N_walks=walks, seed=5, max_steps=1, method="plain")
+    ins = ref.location.reshape(r.location.shape) == 1
+    want, se = ref.mean.reshape(ins.shape)[ins], ref.standard_error.reshape(ins.shape)[ins]
+    close = np.abs(r.mean[ins] - want) <= 1e-9 * np.maximum(1.0, np.abs(want))
+    assert close.mean() >= 0.98, close.mean()
+    if len(set(m.boundary_ids.tolist())) > 1:
+        return
+    f = solver.solve_grid("laplace", *n, N_walks=walks, seed=5, max_steps=1, method="fast64")
+    assert np.array_equal(f.location, r.location)
+    both = np.sqrt(se ** 2 + f.standard_error[ins] ** 2)
+    live = both > 0
+    z = (f.mean[ins] - want)[live] / both[live]
+    assert (np.abs(z) <= 4.5).mean() >= 0.99, np.abs(z).max()

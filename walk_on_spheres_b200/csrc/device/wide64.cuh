@@ -34,6 +34,13 @@ inline bool wide64_usable(const double bbox[6], int dim, float margin) {
     return ext > 1e-9 && mag < 1e9 && static_cast<double>(margin) < 1e-3 * ext;
 }
 
+// Up to this many primitives a lane's own FP64 query (nearest64) beats the
+// warp's when all 32 lanes have one.  FAST_FP64 walk kernel on a B200, ms per
+// thread / by the warp: 2D annulus, 12 M steps: 128 segments 2.26 / 2.98, 200
+// 3.31 / 3.06, 512 4.81 / 3.18; 3D sphere, 1.5 M steps: 64 triangles 2.11 /
+// 2.96, 144 3.60 / 3.21, 256 4.64 / 2.78, 3600 18.8 / 4.38.
+__host__ __device__ __forceinline__ int thread_query_prims(int dim) { return dim == 2 ? 160 : 128; }
+
 // Squared FP64 distance from p to the primitive in binary slot k and its
 // closest point (the leaf test of nearest64).
 template <int DIM>
@@ -120,8 +127,10 @@ __device__ __forceinline__ void visit_clusters(const WideView &w, float px, floa
 // The squared radius that still counts as a candidate once `best2` (a squared
 // FP32 distance, rounded up) has been found.
 __device__ __forceinline__ float candidate_limit(float best2, float margin) {
-    const float r = sqrtf(best2) + 2.0f * margin;
-    return r * r * (1.0f + 0x1p-20f);
+    float r;  // approximate root: the last factor covers its few ulps
+    asm("sqrt.approx.f32 %0, %1;" : "=f"(r) : "f"(best2));
+    r += 2.0f * margin;
+    return r * r * (1.0f + 0x1p-18f);
 }
 
 // Lane minimum of non-negative doubles across the warp.
@@ -134,25 +143,48 @@ __device__ __forceinline__ double warp_min_double(double v) {
         (static_cast<unsigned long long>(mh) << 32) | ml));
 }
 
-// Binary slot of the primitive nearest to (px, py, pz), the same for all 32
-// lanes, which call it with the same point.  Equally near primitives: the
-// lowest slot, except that 2D primitives of different boundaries (a corner
-// where two boundaries meet) are decided by nearest64, so the boundary value
-// is the one the per-thread query picks.
+// The winner among the lanes' candidates (`best`, `slot`: the lane's nearest
+// primitive, slot -1 for none).  Equally near primitives: the lowest slot,
+// except that 2D primitives of different boundaries (a corner where two
+// boundaries meet, in one lane's own candidates when `split`) are decided by
+// nearest64, so the boundary value is the one the per-thread query picks.
 template <int DIM>
-__device__ __forceinline__ int warp_nearest64(const SceneView &s, const WideView &w, double px,
-                                              double py, double pz, float margin) {
+__device__ __forceinline__ int winning_slot(const SceneView &s, double px, double py, double pz,
+                                            double best, int slot, bool split) {
+    constexpr unsigned kAll = 0xffffffffu;
+    const double m = warp_min_double(best);
+    const bool mine = slot >= 0 && best == m;
+    const unsigned ties = __ballot_sync(kAll, mine);
+    if (!ties) return -1;
+    int win = __shfl_sync(kAll, slot, __ffs(ties) - 1);
+    if ((ties & (ties - 1u)) || __any_sync(kAll, mine && split)) {
+        win = static_cast<int>(
+            __reduce_min_sync(kAll, mine ? static_cast<unsigned>(slot) : 0xffffffffu));
+        if constexpr (DIM == 2) {
+            const int bid = s.segid[win].x;
+            if (__any_sync(kAll, mine && (split || s.segid[slot].x != bid))) {
+                win = nearest64<2>(s, px, py, pz, __longlong_as_double(0x7ff0000000000000LL)).slot;
+            }
+        }
+    }
+    return win;
+}
+
+// Binary slot of the primitive nearest to (px, py, pz), every primitive of
+// the visited clusters compared in FP64.  The same for all 32 lanes, which
+// call it with the same point.
+template <int DIM>
+__device__ __forceinline__ int warp_nearest64_full(const SceneView &s, const WideView &w,
+                                                   double px, double py, double pz,
+                                                   float margin) {
     constexpr unsigned kAll = 0xffffffffu;
     const int lane = static_cast<int>(threadIdx.x & 31u);
-    const float fx = static_cast<float>(px), fy = static_cast<float>(py);
-    const float fz = static_cast<float>(pz);
-    // points outside the scene's box (classification) carry larger ulps
-    margin = fmaxf(margin, 4e-6f * fmaxf(fabsf(fx), fmaxf(fabsf(fy), fabsf(fz))));
     double best = __longlong_as_double(0x7ff0000000000000LL);
     int slot = -1;
     bool split = false;  // this lane saw a tie across two boundaries
     float limit = INFINITY, ubest = INFINITY;
-    visit_clusters<DIM>(w, fx, fy, fz, limit, [&](int cluster) {
+    visit_clusters<DIM>(w, static_cast<float>(px), static_cast<float>(py),
+                        static_cast<float>(pz), limit, [&](int cluster) {
         const int ws = cluster * 32 + lane;
         double d2 = __longlong_as_double(0x7ff0000000000000LL);
         if (ws < w.n) {
@@ -173,22 +205,130 @@ __device__ __forceinline__ int warp_nearest64(const SceneView &s, const WideView
             limit = candidate_limit(u, margin);
         }
     });
-    const double m = warp_min_double(best);
-    const bool mine = best == m && slot >= 0;
-    const unsigned ties = __ballot_sync(kAll, mine);
-    if (!ties) return -1;
-    int win = __shfl_sync(kAll, slot, __ffs(ties) - 1);
-    if ((ties & (ties - 1u)) || __any_sync(kAll, mine && split)) {
-        win = static_cast<int>(
-            __reduce_min_sync(kAll, mine ? static_cast<unsigned>(slot) : 0xffffffffu));
-        if constexpr (DIM == 2) {
-            const int bid = s.segid[win].x;
-            if (__any_sync(kAll, mine && (split || s.segid[slot].x != bid))) {
-                win = nearest64<2>(s, px, py, pz, __longlong_as_double(0x7ff0000000000000LL)).slot;
-            }
+    return winning_slot<DIM>(s, px, py, pz, best, slot, split);
+}
+
+// The primitives that can be nearest to a point: binary slots a and, when
+// FP32 distances cannot tell two apart, b (else -1).
+struct Candidates {
+    int a, b;
+};
+
+// This lane's primitive of leaf cluster `cluster`: its squared FP32 distance
+// from p (within the margin of, or above, the true one) and a lower bound of
+// the true squared distance up to the margin.
+//
+// 2D: the two are the same.  Point, vertices and offsets are rounded by at
+// most 2^-23 of the largest coordinate, and the foot's parameter is one
+// quotient, whose error moves the foot by a few 2^-24 of the offset: in all
+// within half the scene's margin.
+//
+// 3D: Eberly's barycentric coordinates divide by det = |e1 x e2|^2.  Their
+// rounding moves the computed closest point inside the triangle by at most
+// about 4 2^-24 (|p - v0| L^4 / det), L the longest edge, and by up to
+// (L^4 / det)^(1/2) times that where it flips the choice of an edge next to
+// an obtuse corner.  A displacement delta from a minimum raises the squared
+// distance by at most delta^2, so the bound subtracts
+// (32 2^-24)^2 k^3 (d^2 + 4 L^2), k = L^4 / det: nothing for ordinary
+// triangles, everything for slivers, which are then compared in FP64.
+template <int DIM>
+__device__ __forceinline__ float lane_distance(const WideView &w, int cluster, float px, float py,
+                                               float pz, float &lower) {
+    if (DIM == 2) {
+        lower = wide_prim_dist<2>(w, cluster, px, py, pz);
+        return lower;
+    }
+    const float *r = w.prim + cluster * (16 * 32) + (threadIdx.x & 31u);
+    float4 rec[4];
+    float *f = reinterpret_cast<float *>(rec);
+#pragma unroll
+    for (int k = 0; k < 16; ++k) f[k] = r[k * 32];
+    const float d = eberly32(px, py, pz, rec);
+    const float a = rec[0].w, b = rec[1].w, c = rec[2].w;
+    const float l2 = fmaxf(a, fmaxf(c, a - 2.0f * b + c));
+    const float k = l2 * l2 * rec[3].y;
+    // fmaxf drops a NaN (a triangle too thin for FP32): bound 0
+    lower = fmaxf(d - 3.7e-12f * (k * k * k) * (d + 4.0f * l2), 0.0f);
+    return d;
+}
+
+// Candidates for the primitive nearest to (px, py, pz), the same for all 32
+// lanes, which call it with the same point; pick_nearest64 decides between
+// them.  FP32 distances choose: a primitive whose lower bound exceeds the
+// smallest distance by more than two margins is not the nearest.  Mostly one
+// primitive is left, sometimes two (next to a vertex of a finely divided
+// curve, or an edge of a surface); the caller forms their FP64 distances for
+// all its lanes at once.  More than two are compared here, and a lane that
+// met two falls back to comparing every primitive in FP64.
+template <int DIM>
+__device__ __forceinline__ Candidates warp_candidates64(const SceneView &s, const WideView &w,
+                                                        double px, double py, double pz) {
+    constexpr unsigned kAll = 0xffffffffu;
+    const int lane = static_cast<int>(threadIdx.x & 31u);
+    const float fx = static_cast<float>(px), fy = static_cast<float>(py);
+    const float fz = static_cast<float>(pz);
+    // points outside the scene's box (classification) carry larger ulps
+    const float margin =
+        fmaxf(w.margin64, 4e-6f * fmaxf(fabsf(fx), fmaxf(fabsf(fy), fabsf(fz))));
+    const float reach = DIM == 2 ? 0.5f * margin : margin;
+    float first = INFINITY, second = INFINITY;  // this lane's two smallest bounds
+    int ws = 0;
+    float limit = INFINITY, ubest = INFINITY;
+    visit_clusters<DIM>(w, fx, fy, fz, limit, [&](int cluster) {
+        float lower;
+        const float d = lane_distance<DIM>(w, cluster, fx, fy, fz, lower);
+        second = fminf(second, fmaxf(first, lower));
+        if (lower < first) {
+            first = lower;
+            ws = cluster * 32 + lane;
+        }
+        const float u = __uint_as_float(__reduce_min_sync(kAll, __float_as_uint(d)));
+        if (u < ubest) {
+            ubest = u;
+            limit = candidate_limit(u, reach);
+        }
+    });
+    const unsigned near = __ballot_sync(kAll, first <= limit && ws < w.n);
+    if (__any_sync(kAll, second <= limit) || near == 0u || !(ubest < INFINITY)) {
+        return Candidates{warp_nearest64_full<DIM>(s, w, px, py, pz, margin), -1};
+    }
+    const int k = __ldg(w.wide2bin + min(ws, w.n - 1));
+    const unsigned rest = near & (near - 1u);
+    const int a = __shfl_sync(kAll, k, __ffs(near) - 1);
+    if (rest == 0u) return Candidates{a, -1};
+    if ((rest & (rest - 1u)) == 0u) return Candidates{a, __shfl_sync(kAll, k, __ffs(rest) - 1)};
+    double best = __longlong_as_double(0x7ff0000000000000LL);
+    const bool mine = (near >> lane) & 1u;
+    double nx, ny, nz;
+    if (mine) best = slot_dist64<DIM>(s, k, px, py, pz, nx, ny, nz);
+    return Candidates{winning_slot<DIM>(s, px, py, pz, best, mine ? k : -1, false), -1};
+}
+
+// The nearest of a point's candidates: its squared FP64 distance, closest
+// point and binary slot.  Equally near: as winning_slot decides.
+template <int DIM>
+__device__ __forceinline__ double pick_nearest64(const SceneView &s, Candidates c, double px,
+                                                 double py, double pz, int &slot, double &nx,
+                                                 double &ny, double &nz) {
+    slot = c.a;
+    double d2 = slot_dist64<DIM>(s, c.a, px, py, pz, nx, ny, nz);
+    if (c.b >= 0) {
+        double bx, by, bz;
+        const double e2 = slot_dist64<DIM>(s, c.b, px, py, pz, bx, by, bz);
+        bool second = e2 < d2 || (e2 == d2 && c.b < c.a);
+        if (DIM == 2 && e2 == d2 && s.segid[c.a].x != s.segid[c.b].x) {
+            second = nearest64<2>(s, px, py, pz, __longlong_as_double(0x7ff0000000000000LL))
+                         .slot == c.b;
+        }
+        if (second) {
+            slot = c.b;
+            d2 = e2;
+            nx = bx;
+            ny = by;
+            nz = bz;
         }
     }
-    return win;
+    return d2;
 }
 
 }  // namespace wosb

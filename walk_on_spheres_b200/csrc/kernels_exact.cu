@@ -328,12 +328,12 @@ __global__ void __launch_bounds__(kExactThreads)
 
 // `per_warp` consecutive points per warp, one per lane; every iteration
 // steps each lane's walk and the whole warp then answers the lanes' queries
-// one after another (warp_nearest64).  A point's walks are serial, so the
+// one after another (warp_candidates64).  A point's walks are serial, so the
 // kernel waits on one step's chain (draw, sine and cosine, query, square
 // root) rather than on issue slots.  Per-thread queries made that chain 30
 // dependent tree nodes long in 32 diverging lanes: 1360 inside points of an
-// annulus of 256 segments, 1000 walks, took 144.8 ms, now 11.9; 0.41 M walks
-// in a blob of 3968 triangles 425 ms, now 11.7 (same results, bit for bit).
+// annulus of 256 segments, 1000 walks, took 144.8 ms, now 10.4; 0.41 M walks
+// in a blob of 3968 triangles 425 ms, now 9.5 (same results, bit for bit).
 template <int DIM, class Eq>
 __global__ void __launch_bounds__(kExactThreads, 4)
     walk_plain_warp_kernel(SceneView s, WideView w, int per_warp, PointSet ps, uint64_t seed,
@@ -356,17 +356,19 @@ __global__ void __launch_bounds__(kExactThreads, 4)
         const bool query = active && k.stepping(eps, max_steps);
         if (query) k.step(eq);
         unsigned pending = __ballot_sync(kAll, query);
-        int slot = -1;
+        Candidates cand{0, -1};
         while (pending) {
             const int j = __ffs(pending) - 1;
             pending &= pending - 1u;
             const double qx = __shfl_sync(kAll, k.p.x, j), qy = __shfl_sync(kAll, k.p.y, j);
             const double qz = DIM == 3 ? __shfl_sync(kAll, k.p.z, j) : 0.0;
-            const int win = warp_nearest64<DIM>(s, w, qx, qy, qz, w.margin64);
-            if (lane == j) slot = win;
+            const Candidates c = warp_candidates64<DIM>(s, w, qx, qy, qz);
+            if (lane == j) cand = c;
         }
         if (query) {
-            k.R = sqrt(slot_dist64<DIM>(s, slot, k.p.x, k.p.y, k.p.z, k.np.x, k.np.y, k.np.z));
+            int slot;
+            k.R = sqrt(pick_nearest64<DIM>(s, cand, k.p.x, k.p.y, k.p.z, slot, k.np.x, k.np.y,
+                                           k.np.z));
             if (DIM == 2) k.bid = s.segid[slot].x;
         }
         if (active && !k.stepping(eps, max_steps)) {
@@ -422,7 +424,9 @@ int blocks_for(long long n, int threads) {
 // / 4.83; 64^2 1.50 / 1.28 / 1.94 / 3.14 / 5.36; 128^2 4.37 / 3.53 / 3.70 /
 // 3.57 / 5.66; 256^2 16.3 / 12.6 / 10.9 / 10.0 / 11.7.  3D sphere of 16 128
 // triangles, 16 walks (queries dominate the step): 24^3 3.88 / 4.15 / 4.37 /
-// 7.31 / 12.1; 40^3 15.4 / 14.4 / 14.7 / 16.5 / 18.3.
+// 7.31 / 12.1; 40^3 15.4 / 14.4 / 14.7 / 16.5 / 18.3 (all with every query
+// compared in FP64; the rule's choices since: 0.82, 1.17, 2.93, 8.16; 3.18,
+// 11.0).
 int points_per_warp(int dim, long long n) {
     if (dim == 3) return n >= 32768 ? 2 : 1;
     int p = 1;

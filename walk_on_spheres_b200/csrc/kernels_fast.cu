@@ -16,7 +16,10 @@
 // position decides termination and supplies the nearest point and
 // boundary id for the boundary value, evaluated in FP64.  Per-walk values are
 // accumulated in FP64 (Welford per lane, Chan's merge across lanes and
-// chunks).  FAST_FP64 runs the same scheduling with FP64 everywhere.
+// chunks).  FAST_FP64 runs the same scheduling with FP64 everywhere; its
+// queries are the warp's (wide64.cuh): the per-thread ones took 32 diverging
+// paths through the binary tree.  Disk of 1024 segments, 22.5 M steps: 18.2 ->
+// 5.4 ms; sphere of 16 128 triangles, 22 M steps: 203 -> 23.6 ms.
 #include <algorithm>
 #include <cmath>
 #include <type_traits>
@@ -69,7 +72,7 @@ __device__ __forceinline__ void fast_task(const FastArgs a, const WideView &wv, 
     T R = R0;
     T sample = T(0), weight = T(1);
     int steps = 0;
-    int slot = -1;                 // FP32: winner of the last query
+    int slot = -1;                 // winner of the last query (FP32: wide slot, FP64: binary)
     V3<double> np64{0.0, 0.0, 0.0};  // FP64: nearest point of the last query
     int bid64 = -1;
     const uint2 pkey = PhiloxStream::key_of(pseed);
@@ -123,6 +126,32 @@ __device__ __forceinline__ void fast_task(const FastArgs a, const WideView &wv, 
                     }
                 }
             } else {
+                need_query = true;
+            }
+        }
+        if constexpr (!kF32) {
+            // FP64 queries by the whole warp, one lane's after another; the
+            // winners' distances then for all lanes at once
+            if (wv.margin64 >= 0.0f && wv.n > thread_query_prims(DIM)) {
+                Candidates cand{0, -1};
+                unsigned pending = __ballot_sync(kFull, need_query);
+                while (pending) {
+                    const int j = __ffs(pending) - 1;
+                    pending &= pending - 1u;
+                    const double qx = __shfl_sync(kFull, static_cast<double>(p.x), j);
+                    const double qy = __shfl_sync(kFull, static_cast<double>(p.y), j);
+                    const double qz =
+                        DIM == 3 ? __shfl_sync(kFull, static_cast<double>(p.z), j) : 0.0;
+                    const Candidates c = warp_candidates64<DIM>(a.s, wv, qx, qy, qz);
+                    if (lane == j) cand = c;
+                }
+                if (need_query) {
+                    R = static_cast<T>(sqrt(pick_nearest64<DIM>(
+                        a.s, cand, static_cast<double>(p.x), static_cast<double>(p.y),
+                        static_cast<double>(p.z), slot, np64.x, np64.y, np64.z)));
+                    bid64 = bid_of<DIM>(a.s, slot);
+                }
+            } else if (need_query) {
                 const Nearest<double> q = nearest64<DIM>(
                     a.s, static_cast<double>(p.x), static_cast<double>(p.y),
                     static_cast<double>(p.z), dinf());
@@ -294,6 +323,14 @@ __device__ __forceinline__ void fast_task(const FastArgs a, const WideView &wv, 
     }
 }
 
+// Blocks per SM of the FP64 walk kernels (80 / 128 registers at 3 / 2): their
+// queries wait on loads and FP64 chains, so resident warps pay, until spills
+// in the 3D queries cost more on small grids.  ms at 1 / 2 / 3: 2D disk of
+// 1024 segments, 73 M steps 33.6 / 19.5 / 16.7; 3D sphere of 16 128 triangles,
+// 22 M steps 41.4 / 23.6 / 20.2, 0.5 M steps 2.23 / 2.34 / 2.53, of 3600, 1.6 M
+// steps 3.95 / 2.72 / 3.17.
+constexpr int min_blocks64(int dim) { return dim == 2 ? 3 : 2; }
+
 template <int DIM>
 __device__ __forceinline__ Laplace<DIM> eq_from(const EqDesc &, Laplace<DIM> *) {
     return Laplace<DIM>{};
@@ -459,7 +496,7 @@ cudaError_t batch_typed(int precision, int hc, const BatchItem *items, int n_ite
             return cudaGetLastError();
         });
     }
-    walk_batch_kernel<DIM, Eq, double, 1, kHeightAny><<<blocks, 256, 0, stream>>>(
+    walk_batch_kernel<DIM, Eq, double, min_blocks64(DIM), kHeightAny><<<blocks, 256, 0, stream>>>(
         items, n_items, n_tasks, queue);
     return cudaGetLastError();
 }
@@ -477,7 +514,7 @@ cudaError_t batch_blocks_typed(int precision, int hc, int &blocks) {
         });
     } else {
         e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-            &per_sm, walk_batch_kernel<DIM, Eq, double, 1, kHeightAny>, 256, 0);
+            &per_sm, walk_batch_kernel<DIM, Eq, double, min_blocks64(DIM), kHeightAny>, 256, 0);
     }
     if (e != cudaSuccess) return e;
     e = cudaGetDevice(&dev);
@@ -620,7 +657,7 @@ cudaError_t launch_fast_typed(const FastArgs &a, const EqDesc &e, int precision,
             return cudaGetLastError();
         });
     } else {
-        auto k = walk_fast_kernel<DIM, Eq, double, 1, kHeightAny>;
+        auto k = walk_fast_kernel<DIM, Eq, double, min_blocks64(DIM), kHeightAny>;
         cudaError_t err = grid_for(k, 0, blocks);
         if (err != cudaSuccess) return err;
         k<<<blocks, plan.threads, 0, stream>>>(a, eq_host<Eq>(e));
