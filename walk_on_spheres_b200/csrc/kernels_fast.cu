@@ -32,6 +32,317 @@ namespace wosb {
 namespace {
 
 
+// Warp merge of the lanes' statistics into the task's partial.
+template <bool kF32>
+__device__ __forceinline__ void write_partial(const FastArgs &a, unsigned long long task,
+                                              const ShiftedSums &acc, int steps_acc, unsigned hits,
+                                              unsigned queries, bool overflow, bool bad) {
+    double n_tot = static_cast<double>(acc.n);
+    double mean_acc, m2_acc;
+    acc.finish(mean_acc, m2_acc);
+    unsigned long long steps_tot = static_cast<unsigned long long>(steps_acc);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        const double nb = __shfl_down_sync(kFull, n_tot, o);
+        const double mb = __shfl_down_sync(kFull, mean_acc, o);
+        const double m2b = __shfl_down_sync(kFull, m2_acc, o);
+        const unsigned long long sb = __shfl_down_sync(kFull, steps_tot, o);
+        const unsigned hb = __shfl_down_sync(kFull, hits, o);
+        chan_merge(n_tot, mean_acc, m2_acc, nb, mb, m2b);
+        steps_tot += sb;
+        hits += hb;
+    }
+    const unsigned any_overflow = __ballot_sync(kFull, overflow);
+    const unsigned any_bad = __ballot_sync(kFull, bad);
+    if ((threadIdx.x & 31) == 0) {
+        if (any_bad) atomicOr(&a.ctr->error_flags, kErrBadState);
+        TaskPartial tp;
+        tp.n = n_tot;
+        tp.mean = mean_acc;
+        tp.m2 = m2_acc;
+        tp.steps = static_cast<double>(steps_tot);
+        tp.queries = kF32 ? static_cast<double>(queries) : static_cast<double>(steps_tot);
+        tp.hits = hits;
+        tp.pad = 0;
+        a.partials[task] = tp;
+        if (any_overflow) atomicOr(&a.ctr->error_flags, kErrRejectionCap);
+    }
+}
+
+// Walks that wait in shared memory, kPool slots per warp, one array per field.
+// Slots from 0 up hold walks whose last step needs a closest-point query,
+// slots from kPool - 1 down walks to be resumed with the radius found.
+constexpr int kPool = 64;
+
+template <int DIM, class Eq>
+struct WalkPool {
+    static constexpr int kFields = 5 + (DIM == 3) + (Eq::kSource ? 1 : 0) +
+                                   (Eq::kScreening ? 1 : 0);
+    unsigned *f;
+    __device__ __forceinline__ float &real(int field, int i) {
+        return reinterpret_cast<float *>(f)[field * kPool + i];
+    }
+    __device__ __forceinline__ float &radius(int i) { return real(4, i); }
+    __device__ __forceinline__ void put(int i, V3<float> p, float sample, float weight, int steps,
+                                        int walk) {
+        f[i] = static_cast<unsigned>(steps);
+        f[kPool + i] = static_cast<unsigned>(walk);
+        real(2, i) = p.x;
+        real(3, i) = p.y;
+        int k = 5;
+        if constexpr (DIM == 3) real(k++, i) = p.z;
+        if constexpr (Eq::kSource) real(k++, i) = sample;
+        if constexpr (Eq::kScreening) real(k++, i) = weight;
+    }
+    __device__ __forceinline__ void get(int i, V3<float> &p, float &sample, float &weight,
+                                        int &steps, int &walk) {
+        steps = static_cast<int>(f[i]);
+        walk = static_cast<int>(f[kPool + i]);
+        p = V3<float>{real(2, i), real(3, i), 0.0f};
+        sample = 0.0f;
+        weight = 1.0f;
+        int k = 5;
+        if constexpr (DIM == 3) p.z = real(k++, i);
+        if constexpr (Eq::kSource) sample = real(k++, i);
+        if constexpr (Eq::kScreening) weight = real(k++, i);
+    }
+};
+
+// Which walk kernels put walks aside: FAST_FP32 ones, except on lane-scan
+// scenes, where a query is one short scan that every lane runs at every step.
+// Measured there against fast_task: laplace and poisson 3-4% faster with the
+// pool, screened_poisson 5% and the transient plate 11% slower (their
+// rejection samplers fill the step, and the pool costs registers).
+template <typename T, int HC>
+constexpr bool kPooled = std::is_same<T, float>::value && HC != kLaneScan;
+
+// One FAST_FP32 task: walks [c*chunk, min(N, (c+1)*chunk)) of point pidx,
+// written to a.partials[task].  The lanes only take steps; a walk whose step
+// needs a query (near the boundary: mostly its last step) is put aside in
+// the warp's pool, and its lane steps another walk in the next iteration.
+// When 32 walks wait, the warp answers them together, one per lane: list
+// scan or cooperative query, shell test, FP64 re-projection, boundary value
+// and statistics; walks that go on return to the lanes.  So both halves run
+// with (nearly) all lanes.  A walk's draws depend on its own index and step
+// alone, so its path is the same wherever and whenever its steps run.
+//
+// The pool never overflows: a new walk starts only when no walk waits to be
+// resumed, with at most 31 walks waiting for a query and 31 in other lanes;
+// so at most 63 are under way.
+template <int DIM, class Eq, int HC>
+__device__ __forceinline__ void fast_task32(const FastArgs a, const WideView &wv, const Eq &eq,
+                                            unsigned long long task, long long pidx, int c,
+                                            unsigned *s_pool) {
+    const int lane = threadIdx.x & 31;
+    const unsigned lt_mask = (1u << lane) - 1u;
+    WalkPool<DIM, Eq> pool{s_pool};
+
+    double x0, y0, z0;
+    uint64_t linear;
+    point_at(a.ps, pidx, x0, y0, z0, linear);
+    const uint64_t pseed = point_seed(a.seed, linear);
+    const V3<float> p0{static_cast<float>(x0), static_cast<float>(y0), static_cast<float>(z0)};
+    const double r0 = a.start[pidx].radius;
+    const float R0 = static_cast<float>(r0);
+    const int w0 = c * a.chunk;
+    const int w1 = min(a.n_walks, w0 + a.chunk);
+
+    int steps_acc = 0;
+    ShiftedSums acc;
+    unsigned hits = 0;
+    // BVH closest-point queries of this task (warp-uniform).  At most
+    // chunk * max_steps < 2^32 (set_chunk).
+    unsigned queries = 0;
+    bool overflow = false;
+    bool bad = false;  // a closest-point query found no primitive
+
+    if (!(r0 > a.eps)) {
+        // the start point is inside the shell: every walk ends there
+        const StartRecord st = a.start[pidx];
+        const double value = eq.boundary(V3<double>{st.nx, st.ny, st.nz}, st.boundary_id);
+        for (int w = w0 + lane; w < w1; w += 32) acc.add(value);
+        write_partial<true>(a, task, acc, 0, 0u, 0u, false, false);
+        return;
+    }
+
+    bool active = false;
+    int walk = 0, steps = 0;
+    V3<float> p = p0;
+    float R = R0, sample = 0.0f, weight = 1.0f;
+    int next = w0;    // next new walk
+    int waiting = 0;  // walks waiting for a query
+    int resume = 0;   // walks waiting for a lane
+    const uint2 pkey = PhiloxStream::key_of(pseed);
+
+    for (;;) {
+        // lanes without a walk take one: a resumed walk, else a new one
+        const unsigned empty = __ballot_sync(kFull, !active);
+        if (empty) {
+            if (!active) {
+                const int rank = __popc(empty & lt_mask);
+                if (rank < resume) {
+                    const int i = kPool - resume + rank;
+                    pool.get(i, p, sample, weight, steps, walk);
+                    R = pool.radius(i);
+                    active = true;
+                } else {
+                    walk = next + rank - resume;
+                    active = walk < w1;
+                    p = p0;
+                    R = R0;
+                    sample = 0.0f;
+                    weight = 1.0f;
+                    steps = 0;
+                }
+            }
+            const int taken = __popc(empty);
+            next = min(next + max(taken - resume, 0), w1);
+            resume = max(resume - taken, 0);
+            __syncwarp();
+        }
+        // one step of every walk in flight
+        bool defer = false;
+        if (active) {
+            FastRng<float> rng(pkey, static_cast<uint32_t>(walk));
+            rng.begin_step(steps);
+            p = walk_body<DIM, false, float>(eq, p, R, sample, weight, rng, rng, overflow);
+            ++steps;
+            defer = true;
+            // away from the shell a lattice lower bound is a valid (smaller)
+            // radius and spares the exact query; the step that reaches the
+            // cap queries, for its nearest point
+            if (wv.gd != nullptr && steps < a.max_steps) {
+                const LatticeSample ls = lattice_sample<DIM>(wv, p.x, p.y, DIM == 3 ? p.z : 0.0f);
+                const float gb = (ls.d - ls.r) * a.shrink;
+                if (ls.d >= wv.gratio * ls.r && gb > 0.0f && gb * gb > a.shell2) {
+                    R = gb;
+                    defer = false;
+                }
+            }
+        }
+        const unsigned put = __ballot_sync(kFull, defer);
+        if (put) {
+            if (defer) {
+                const int i = waiting + __popc(put & lt_mask);
+                pool.put(i, p, sample, weight, steps, walk);
+                active = false;
+            }
+            waiting += __popc(put);
+            __syncwarp();
+        }
+        const bool idle = !__any_sync(kFull, active);
+        if (idle && waiting == 0 && resume == 0 && next >= w1) break;
+        if (waiting < 32 && !(idle && next >= w1 && resume == 0)) continue;
+
+        // ---- the waiting walks' queries and endings, one walk per lane
+        const int m = min(waiting, 32);
+        waiting -= m;
+        const bool has = lane < m;
+        V3<float> q{0.0f, 0.0f, 0.0f};
+        float qR = 0.0f, qsample = 0.0f, qweight = 1.0f;
+        int qsteps = 0, qwalk = 0, slot = -1;
+        int packed = -1;  // the node's candidate list, if any
+        if (has) {
+            pool.get(waiting + lane, q, qsample, qweight, qsteps, qwalk);
+            if (wv.gl != nullptr && qsteps < a.max_steps) {
+                const LatticeSample ls = lattice_sample<DIM>(wv, q.x, q.y, DIM == 3 ? q.z : 0.0f);
+                if (ls.d <= a.list_t) {
+                    const int2 e = __ldg(wv.gl + ls.node);
+                    packed = DIM == 3 && e.x >= 0 ? list_prefix(wv, e, ls.r) : e.x;
+                }
+            }
+        }
+        __syncwarp();
+        const bool want = has && packed >= 0;
+        float qbest = 0.0f;
+        if constexpr (DIM == 2) {
+            if (want) {
+                const WideResult r =
+                    list_nearest<DIM>(wv, list_of(wv, packed), list_length(packed), q.x, q.y,
+                                      0.0f);
+                qbest = r.best;
+                slot = r.slot;
+            }
+        } else if (__any_sync(kFull, want)) {
+            const WideResult r =
+                warp_list_nearest<DIM>(wv, want, packed, q.x, q.y, q.z);
+            if (want) {
+                qbest = r.best;
+                slot = r.slot;
+            }
+        }
+        // no list: the warp resolves each such query together
+        unsigned pending = __ballot_sync(kFull, has && packed < 0);
+        while (pending) {
+            const int j = __ffs(pending) - 1;
+            pending &= pending - 1u;
+            const float qx = __shfl_sync(kFull, q.x, j);
+            const float qy = __shfl_sync(kFull, q.y, j);
+            const float qz = DIM == 3 ? __shfl_sync(kFull, q.z, j) : 0.0f;
+            const WideResult r = wide_nearest<DIM, HC>(wv, qx, qy, qz, a.keep, a.exact2);
+            if (lane == j) {
+                qbest = r.best;
+                slot = r.slot;
+            }
+        }
+        queries += m;
+        const float r = sqrtf(qbest);
+        qR = qbest > a.shell2 ? r * a.shrink : r;
+        bool go_on = false;
+        if (has) {
+            bool stop = false;
+            V3<double> np{0.0, 0.0, 0.0};
+            int bid = -1;
+            if (qR * qR <= a.shell2) {
+                // epsilon shell: FP64 re-projection onto the nearest primitive
+                // (a query that found none is a broken walk: flag it, stop)
+                if (slot < 0) {
+                    bad = true;
+                    stop = true;
+                } else {
+                    const double d2 = reproject64_sq<DIM>(
+                        a.s, wv.wide2bin[slot], static_cast<double>(q.x),
+                        static_cast<double>(q.y), static_cast<double>(q.z), np, bid);
+                    if (d2 <= a.eps * a.eps) {
+                        stop = true;
+                    } else {
+                        qR = static_cast<float>(sqrt(d2));
+                    }
+                }
+            }
+            if (!stop && qsteps >= a.max_steps) {
+                // step cap: finish at the nearest boundary point
+                // (include/wos/wos.hpp:129-137)
+                ++hits;
+                stop = true;
+                if (slot < 0) {
+                    bad = true;
+                } else {
+                    reproject64<DIM>(a.s, wv.wide2bin[slot], static_cast<double>(q.x),
+                                     static_cast<double>(q.y), static_cast<double>(q.z), np, bid);
+                }
+            }
+            if (stop) {
+                acc.add(static_cast<double>(qsample) +
+                        static_cast<double>(qweight) * eq.boundary(np, bid));
+                steps_acc += qsteps;
+            }
+            go_on = !stop;
+        }
+        const unsigned back = __ballot_sync(kFull, go_on);
+        if (back) {
+            if (go_on) {
+                const int i = kPool - 1 - resume - __popc(back & lt_mask);
+                pool.put(i, q, qsample, qweight, qsteps, qwalk);
+                pool.radius(i) = qR;
+            }
+            resume += __popc(back);
+            __syncwarp();
+        }
+    }
+    write_partial<true>(a, task, acc, steps_acc, hits, queries, overflow, bad);
+}
+
 // One task: walks [c*chunk, min(N, (c+1)*chunk)) of point pidx, written to
 // a.partials[task] as Welford statistics.
 template <int DIM, class Eq, typename T, int HC>
@@ -290,37 +601,7 @@ __device__ __forceinline__ void fast_task(const FastArgs a, const WideView &wv, 
         }
     }
 
-    // warp merge of the lanes' statistics
-    double n_tot = static_cast<double>(acc.n);
-    double mean_acc, m2_acc;
-    acc.finish(mean_acc, m2_acc);
-    unsigned long long steps_tot = static_cast<unsigned long long>(steps_acc);
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        const double nb = __shfl_down_sync(kFull, n_tot, o);
-        const double mb = __shfl_down_sync(kFull, mean_acc, o);
-        const double m2b = __shfl_down_sync(kFull, m2_acc, o);
-        const unsigned long long sb = __shfl_down_sync(kFull, steps_tot, o);
-        const unsigned hb = __shfl_down_sync(kFull, hits, o);
-        chan_merge(n_tot, mean_acc, m2_acc, nb, mb, m2b);
-        steps_tot += sb;
-        hits += hb;
-    }
-    const unsigned any_overflow = __ballot_sync(kFull, overflow);
-    const unsigned any_bad = __ballot_sync(kFull, bad);
-    if (lane == 0) {
-        if (any_bad) atomicOr(&a.ctr->error_flags, kErrBadState);
-        TaskPartial tp;
-        tp.n = n_tot;
-        tp.mean = mean_acc;
-        tp.m2 = m2_acc;
-        tp.steps = static_cast<double>(steps_tot);
-        tp.queries = kF32 ? static_cast<double>(queries) : static_cast<double>(steps_tot);
-        tp.hits = hits;
-        tp.pad = 0;
-        a.partials[task] = tp;
-        if (any_overflow) atomicOr(&a.ctr->error_flags, kErrRejectionCap);
-    }
+    write_partial<kF32>(a, task, acc, steps_acc, hits, queries, overflow, bad);
 }
 
 // Blocks per SM of the FP64 walk kernels (80 / 128 registers at 3 / 2): their
@@ -353,6 +634,8 @@ __global__ void __launch_bounds__(256, MIN_BLOCKS) walk_fast_kernel(FastArgs a, 
     constexpr bool kF32 = std::is_same<T, float>::value;
     extern __shared__ float4 smem[];
     __shared__ int s_off[8];
+    __shared__ unsigned s_pool[kPooled<T, HC> ? 8 : 1]
+                              [kPooled<T, HC> ? WalkPool<DIM, Eq>::kFields * kPool : 1];
     if (threadIdx.x < 8) s_off[threadIdx.x] = a.w.off[threadIdx.x];
     WideView wv = a.w;
     wv.off = s_off;
@@ -381,7 +664,11 @@ __global__ void __launch_bounds__(256, MIN_BLOCKS) walk_fast_kernel(FastArgs a, 
         const long long pidx = static_cast<long long>(task / a.chunks);
         const int c = static_cast<int>(task % a.chunks);
         if (a.location[pidx] != 1) continue;
-        fast_task<DIM, Eq, T, HC>(a, wv, eq, task, pidx, c);
+        if constexpr (kPooled<T, HC>) {
+            fast_task32<DIM, Eq, HC>(a, wv, eq, task, pidx, c, s_pool[threadIdx.x >> 5]);
+        } else {
+            fast_task<DIM, Eq, T, HC>(a, wv, eq, task, pidx, c);
+        }
     }
 }
 
@@ -394,6 +681,8 @@ __global__ void __launch_bounds__(256, MIN_BLOCKS)
     walk_batch_kernel(const BatchItem *__restrict__ items, int n_items, long long n_tasks,
                       unsigned long long *queue) {
     __shared__ int s_off[8][8];  // per warp: wide-tree offsets of the warp's current item
+    __shared__ unsigned s_pool[kPooled<T, HC> ? 8 : 1]
+                              [kPooled<T, HC> ? WalkPool<DIM, Eq>::kFields * kPool : 1];
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
     int cur = -1;
@@ -423,7 +712,13 @@ __global__ void __launch_bounds__(256, MIN_BLOCKS)
         WideView wv = it.a.w;
         wv.off = s_off[warp];
         const Eq eq = eq_from(it.eq, static_cast<Eq *>(nullptr));
-        fast_task<DIM, Eq, T, HC>(it.a, wv, eq, static_cast<unsigned long long>(local), pidx, c);
+        if constexpr (kPooled<T, HC>) {
+            fast_task32<DIM, Eq, HC>(it.a, wv, eq, static_cast<unsigned long long>(local), pidx, c,
+                                     s_pool[warp]);
+        } else {
+            fast_task<DIM, Eq, T, HC>(it.a, wv, eq, static_cast<unsigned long long>(local), pidx,
+                                      c);
+        }
     }
 }
 
@@ -646,7 +941,8 @@ cudaError_t launch_fast_typed(const FastArgs &a, const EqDesc &e, int precision,
             // 3 for the generic one
             constexpr int kMinBlocks = (HC == kHeightUpTo2 || HC == kHeight3) ? 4 : 3;
             auto k = walk_fast_kernel<DIM, Eq, float, kMinBlocks, HC>;
-            if (plan.smem_bytes > 48 * 1024) {
+            // (the walk pools are static shared memory beside it)
+            if (plan.smem_bytes > 0) {
                 cudaError_t err = cudaFuncSetAttribute(
                     k, cudaFuncAttributeMaxDynamicSharedMemorySize, plan.smem_bytes);
                 if (err != cudaSuccess) return err;
