@@ -15,6 +15,8 @@
 // they round identically), the fast path with float.  Random draws come from
 // an Rng with unit() in [0, 1) and unit_open() in (0, 1).
 #pragma once
+#include <type_traits>
+
 #include "special.cuh"
 
 namespace wosb {
@@ -42,6 +44,15 @@ __device__ __forceinline__ T harmonic_y5(T x, T y, T z) {
     const T y5m3 = (T(8) * z * z - r_sq) * y * (T(3) * x * x - y * y);
     return y50 + T(4) * y5m3;
 }
+
+// a^2 + b^2 of the disk tests that decide draws.  In FP32 the rounding is
+// spelled out (b^2 fused onto the rounded a^2): left to the compiler, the
+// fused product can change with the code around it, and a test that falls the
+// other way in the last bit changes a walk's draws.
+__device__ __forceinline__ float sum_of_squares(float a, float b) {
+    return __fmaf_rn(b, b, __fmul_rn(a, a));
+}
+__device__ __forceinline__ double sum_of_squares(double a, double b) { return a * a + b * b; }
 
 template <int DIM, typename T>
 __device__ __forceinline__ T dist(V3<T> a, V3<T> b) {
@@ -200,26 +211,68 @@ __device__ __forceinline__ T sc_weight_2d(T alpha, T R) {
     }
     return exp(-log_i0(x));
 }
+
+// What the 2D screened kernels need of a ball B(R): X = alpha R and ln I0(X),
+// which a step forms once and shares between the proposals of its rejection
+// sampler, the Green mass and the weight (they are the larger part of each;
+// FP64: a series or a 27-node quadrature), and for the sampler's test
+// ln K0(X) (FP64) or, in FP32, an approximate K0(X) / I0(X) (X < 2) or
+// ln K0(X) - ln I0(X).
 template <typename T>
-__device__ __forceinline__ T sc_green_2d(T alpha, T R, T r) {
-    if (!(r > T(0)) || r > R || R <= T(0)) return T(NAN);
-    if (r == R) return T(0);
-    const T x = alpha * r, X = alpha * R;
-    if (X < T(1e-5)) return pg_green_2d(R, r);
+struct ScreenedBall {
+    T R, X, li, k;
+};
+template <typename T>
+__device__ __forceinline__ ScreenedBall<T> sc_ball_2d(T alpha, T R);
+template <>
+__device__ __forceinline__ ScreenedBall<double> sc_ball_2d<double>(double alpha, double R) {
+    const double X = alpha * R;
+    return ScreenedBall<double>{R, X, log_i0(X), log_k0(X)};
+}
+template <>
+__device__ __forceinline__ ScreenedBall<float> sc_ball_2d<float>(float alpha, float R) {
+    const float X = alpha * R;
+    ScreenedBall<float> b{R, X, log_i0(X), 0.0f};
+    if (X < 2.0f) {
+        const float i0 = as_i0_small(X);
+        b.k = __fdividef(quick_k0_small(X, i0), i0);
+    } else {
+        b.k = quick_log_k0(X) - b.li;
+    }
+    return b;
+}
+__device__ __forceinline__ double sc_ball_log_k0(const ScreenedBall<double> &b) { return b.k; }
+__device__ __forceinline__ float sc_ball_log_k0(const ScreenedBall<float> &b) {
+    return log_k0(b.X);
+}
+template <typename T>
+__device__ __forceinline__ T sc_weight_2d(const ScreenedBall<T> &b) {
+    if (b.X == T(0)) return T(1);
+    if (b.X < T(1e-3)) {
+        const T x2 = b.X * b.X;
+        return T(1) - x2 / T(4) + T(3) * x2 * x2 / T(64);
+    }
+    return exp(-b.li);
+}
+template <typename T>
+__device__ __forceinline__ T sc_green_2d(T alpha, const ScreenedBall<T> &b, T r) {
+    if (!(r > T(0)) || r > b.R || b.R <= T(0)) return T(NAN);
+    if (r == b.R) return T(0);
+    const T x = alpha * r;
+    if (b.X < T(1e-5)) return pg_green_2d(b.R, r);
     const T la = log_k0(x);
-    const T lb = log_i0(x) + log_k0(X) - log_i0(X);
+    const T lb = log_i0(x) + sc_ball_log_k0(b) - b.li;
     T delta = lb - la;
     if (delta > T(0)) delta = T(0);
     return exp(la) * (-expm1(delta)) / (T(2) * T(kPi));
 }
 template <typename T>
-__device__ __forceinline__ T sc_mass_2d(T alpha, T R) {
-    const T x = alpha * R;
-    if (x < T(1e-3)) {
-        const T x2 = x * x;
-        return R * R * (T(1) / T(4) - T(3) * x2 / T(64) + T(19) * x2 * x2 / T(2304));
+__device__ __forceinline__ T sc_mass_2d(T alpha, const ScreenedBall<T> &b) {
+    if (b.X < T(1e-3)) {
+        const T x2 = b.X * b.X;
+        return b.R * b.R * (T(1) / T(4) - T(3) * x2 / T(64) + T(19) * x2 * x2 / T(2304));
     }
-    return -expm1(-log_i0(x)) / (alpha * alpha);
+    return -expm1(-b.li) / (alpha * alpha);
 }
 template <typename T>
 __device__ __forceinline__ T sc_weight_3d(T alpha, T R) {
@@ -267,25 +320,70 @@ __device__ __forceinline__ T sc_normal(Rng &rng) {
 // are never used up in practice).
 constexpr int kRejectionCap = 4096;
 
+// Acceptance probability of a proposed radius r < R.
+template <typename T>
+__device__ __forceinline__ T sc_acceptance_2d(T alpha, const ScreenedBall<T> &b, T r) {
+    if (b.X < T(2)) {
+        const T proposal = pg_green_2d(b.R, r);
+        return sc_green_2d(alpha, b, r) / proposal;
+    }
+    const T x = alpha * r;
+    const T lr = log_i0(x) + sc_ball_log_k0(b) - b.li - log_k0(x);
+    return -expm1((lr < T(0)) ? lr : T(0));
+}
+
+// Whether u < clamp_probability(sc_acceptance_2d(r)).  FP32: the probability
+// (K0(x) - I0(x) K0(X)/I0(X)) / ln(R/r), or 1 - (I0(x)/K0(x)) (K0(X)/I0(X)) in
+// a large ball, is first formed with approximate instructions (about 45 of
+// them against 230).  The rounding of either form is below a fifth of `tol`:
+// 1e-6 of the terms' sizes, in a large ball a few ulps of exponents near X.
+// Only a u that lies closer than that (about one proposal in 10^4) is
+// decided by sc_acceptance_2d, so every decision is the one it makes.
+__device__ __forceinline__ bool sc_accepts_2d(double alpha, const ScreenedBall<double> &b,
+                                              double r, double u) {
+    return u < clamp_probability(sc_acceptance_2d(alpha, b, r));
+}
+__device__ __forceinline__ bool sc_accepts_2d(float alpha, const ScreenedBall<float> &b, float r,
+                                              float u) {
+    const float x = alpha * r;
+    float gap, tol;  // accepted where gap > 0
+    if (b.X < 2.0f) {
+        const float i0 = as_i0_small(x);
+        const float k0 = quick_k0_small(x, i0);
+        const float l = __logf(__fdividef(b.R, r));
+        gap = k0 - i0 * b.k - u * l;
+        // below 1e-5 the probability is 1 by another formula
+        tol = b.X < 1e-5f ? INFINITY : 1e-5f * (1.0f + k0 + l);
+    } else {
+        const float e = __expf(quick_log_i0(x) - quick_log_k0(x) + b.k);
+        gap = (1.0f - u) - e;
+        tol = e * (1e-5f + 4e-6f * b.X) + 1e-6f;
+    }
+    // NaN and infinities fail the comparison
+    if (fabsf(gap) > tol && tol > 0.0f) return gap > 0.0f;
+    return u < clamp_probability(sc_acceptance_2d(alpha, b, r));
+}
+
+// One proposal of the 2D sampler: its radius, and whether it is accepted.
 template <typename T, class Rng>
-__device__ __forceinline__ T sc_sample_radius_2d(T alpha, T R, Rng &rng, bool &overflow) {
-    const T X = alpha * R;
-    T r = R * T(0.5);
+__device__ __forceinline__ bool sc_try_radius_2d(T alpha, const ScreenedBall<T> &b, Rng &rng,
+                                                 T &r) {
+    if (b.X < T(2)) {
+        r = pg_sample_radius_2d(b.R, rng);
+    } else {
+        const T time = -log(rng.unit_open()) / (alpha * alpha);
+        r = sqrt(T(-4) * time * log(rng.unit_open()));
+        if (r >= b.R) return false;
+    }
+    return sc_accepts_2d(alpha, b, r, rng.unit());
+}
+
+template <typename T, class Rng>
+__device__ __forceinline__ T sc_sample_radius_2d(T alpha, const ScreenedBall<T> &b, Rng &rng,
+                                                 bool &overflow) {
+    T r = b.R * T(0.5);
     for (int it = 0; it < kRejectionCap; ++it) {
-        T acc;
-        if (X < T(2)) {
-            r = pg_sample_radius_2d(R, rng);
-            const T proposal = pg_green_2d(R, r);
-            acc = sc_green_2d(alpha, R, r) / proposal;
-        } else {
-            const T time = -log(rng.unit_open()) / (alpha * alpha);
-            r = sqrt(T(-4) * time * log(rng.unit_open()));
-            if (r >= R) continue;
-            const T x = alpha * r;
-            const T lr = log_i0(x) + log_k0(X) - log_i0(X) - log_k0(x);
-            acc = -expm1((lr < T(0)) ? lr : T(0));
-        }
-        if (rng.unit() < clamp_probability(acc)) return r;
+        if (sc_try_radius_2d(alpha, b, rng, r)) return r;
     }
     overflow = true;
     return r;
@@ -358,7 +456,7 @@ struct Poisson {
     __device__ bool may_intersect(V3<T> c, T R) const {
         const T dx = c.x - T(0), dy = c.y - T(0);
         const T reach = R + T(0.15);
-        return dx * dx + dy * dy <= reach * reach;
+        return sum_of_squares(dx, dy) <= reach * reach;
     }
     template <typename T>
     __device__ T source(V3<T> p) const {
@@ -388,7 +486,7 @@ struct Poisson {
 // and the degree-5 harmonic boundary data.
 template <int DIM>
 struct Screened {
-    static constexpr bool kSource = (DIM == 2), kScreening = true;
+    static constexpr bool kSource = (DIM == 2), kScreening = true, kBalls = (DIM == 2);
     int mode;
     double alpha;
     template <typename T>
@@ -400,7 +498,7 @@ struct Screened {
     __device__ bool may_intersect(V3<T> c, T R) const {
         const T dx = c.x - T(0.45), dy = c.y - T(0);
         const T reach = R + T(0.5);
-        return dx * dx + dy * dy <= reach * reach;
+        return sum_of_squares(dx, dy) <= reach * reach;
     }
     template <typename T>
     __device__ T source(V3<T> p) const {
@@ -410,17 +508,17 @@ struct Screened {
     template <typename T>
     __device__ T green(T R, T r) const {
         const T a = static_cast<T>(alpha);
-        return DIM == 2 ? sc_green_2d(a, R, r) : sc_green_3d(a, R, r);
+        return DIM == 2 ? sc_green_2d(a, sc_ball_2d(a, R), r) : sc_green_3d(a, R, r);
     }
     template <typename T>
     __device__ T green_mass(T R) const {
         const T a = static_cast<T>(alpha);
-        return DIM == 2 ? sc_mass_2d(a, R) : sc_mass_3d(a, R);
+        return DIM == 2 ? sc_mass_2d(a, sc_ball_2d(a, R)) : sc_mass_3d(a, R);
     }
     template <typename T, class Rng>
     __device__ T green_radius(T R, Rng &rng, bool &overflow) const {
         const T a = static_cast<T>(alpha);
-        return DIM == 2 ? sc_sample_radius_2d(a, R, rng, overflow)
+        return DIM == 2 ? sc_sample_radius_2d(a, sc_ball_2d(a, R), rng, overflow)
                         : sc_sample_radius_3d(a, R, rng, overflow);
     }
     template <typename T>
@@ -472,7 +570,21 @@ struct TransientDesc {
     double xmin, xmax, ymin, ymax;
     int cubic;             // 1: cubic Lagrange history interpolation, 0: bilinear
     int pad;
+    // the quotients of transient_source, for transient_source_quick (set_quotients)
+    double a2, gx, gy, isx, isy, heat, ik;
 };
+
+inline void set_quotients(TransientDesc &t) {
+    t.a2 = t.alpha * t.alpha;
+    t.gx = static_cast<double>(t.nx - 1) / (t.xmax - t.xmin);
+    t.gy = static_cast<double>(t.ny - 1) / (t.ymax - t.ymin);
+    t.isx = 1.0 / t.sx;
+    t.isy = 1.0 / t.sy;
+    t.ik = 1.0 / t.conductivity;
+    t.heat = t.kind == 2 && t.fraction > 0.0
+                 ? t.fraction * t.power / (t.thickness * t.ix * t.iy * t.conductivity)
+                 : 0.0;
+}
 
 __device__ __forceinline__ double clamp_ref(double v, double lo, double hi) {
     return v < lo ? lo : (hi < v ? hi : v);  // std::clamp
@@ -551,9 +663,58 @@ __device__ __forceinline__ double transient_source(const TransientDesc &t, doubl
     return previous + heat;
 }
 
+// transient_source with its divisions formed once per step on the host, for
+// the FP32 walks: the same FP64 value to a few ulps (they round it to FP32).
+// Ten FP64 divisions took most of a step on the plate.
+__device__ __forceinline__ double gauss_quick(double dx, double dy) {
+    return exp(-0.5 * (dx * dx + dy * dy));
+}
+__device__ __forceinline__ double transient_source_quick(const TransientDesc &t, double x,
+                                                         double y) {
+    const double gx = fmin(fmax((x - t.xmin) * t.gx, 0.0), static_cast<double>(t.nx - 1));
+    const double gy = fmin(fmax((y - t.ymin) * t.gy, 0.0), static_cast<double>(t.ny - 1));
+    double v = 0.0;
+    if (t.cubic && t.nx >= 4 && t.ny >= 4) {
+        const int ix = min(max(static_cast<int>(gx) - 1, 0), t.nx - 4);
+        const int iy = min(max(static_cast<int>(gy) - 1, 0), t.ny - 4);
+        // Lagrange weights: products of the distances to the other nodes
+        const double c = gx - static_cast<double>(ix), d = gy - static_cast<double>(iy);
+        const double c1 = c - 1.0, c2 = c - 2.0, c3 = c - 3.0;
+        const double d1 = d - 1.0, d2 = d - 2.0, d3 = d - 3.0;
+        const double wx[4] = {c1 * c2 * c3 * (-1.0 / 6.0), c * c2 * c3 * 0.5,
+                              c * c1 * c3 * -0.5, c * c1 * c2 * (1.0 / 6.0)};
+        const double wy[4] = {d1 * d2 * d3 * (-1.0 / 6.0), d * d2 * d3 * 0.5,
+                              d * d1 * d3 * -0.5, d * d1 * d2 * (1.0 / 6.0)};
+        const double *row = t.prev + ix * t.ny + iy;
+#pragma unroll
+        for (int di = 0; di < 4; ++di, row += t.ny) {
+            v += wx[di] * (wy[0] * row[0] + wy[1] * row[1] + wy[2] * row[2] + wy[3] * row[3]);
+        }
+    } else {
+        const int i0 = static_cast<int>(gx), j0 = static_cast<int>(gy);
+        const int i1 = min(i0 + 1, t.nx - 1), j1 = min(j0 + 1, t.ny - 1);
+        const double tx = gx - static_cast<double>(i0), ty = gy - static_cast<double>(j0);
+        const double lower = (1.0 - tx) * field_at(t, i0, j0) + tx * field_at(t, i1, j0);
+        const double upper = (1.0 - tx) * field_at(t, i0, j1) + tx * field_at(t, i1, j1);
+        v = (1.0 - ty) * lower + ty * upper;
+    }
+    if (t.kind == 0) return t.a2 * v;
+    double f = t.a2 * fmax(v, 0.0);
+    if (t.kind == 3) {
+        double value = 0.0;
+        for (int k = 0; k < t.moving; ++k) {
+            value += t.mcoef[k] * gauss_quick((x - t.mx[k]) * t.isx, (y - t.my[k]) * t.isy);
+        }
+        f += value * t.ik;
+    } else if (t.heat != 0.0) {
+        f += t.heat * gauss_quick((x - t.cx) * t.isx, (y - t.cy) * t.isy);
+    }
+    return f;
+}
+
 template <int DIM>
 struct Transient {
-    static constexpr bool kSource = true, kScreening = true;
+    static constexpr bool kSource = true, kScreening = true, kBalls = true;
     int mode;  // always kGreen: screened Green source samples
     double alpha;
     const TransientDesc *t;
@@ -563,16 +724,27 @@ struct Transient {
     __device__ bool may_intersect(V3<T>, T) const { return true; }
     template <typename T>
     __device__ T source(V3<T> p) const {
-        return static_cast<T>(transient_source(*t, static_cast<double>(p.x),
-                                               static_cast<double>(p.y)));
+        if constexpr (std::is_same<T, float>::value) {
+            return static_cast<float>(transient_source_quick(*t, static_cast<double>(p.x),
+                                                             static_cast<double>(p.y)));
+        } else {
+            return transient_source(*t, p.x, p.y);
+        }
     }
     template <typename T>
-    __device__ T green(T R, T r) const { return sc_green_2d(static_cast<T>(alpha), R, r); }
+    __device__ T green(T R, T r) const {
+        const T a = static_cast<T>(alpha);
+        return sc_green_2d(a, sc_ball_2d(a, R), r);
+    }
     template <typename T>
-    __device__ T green_mass(T R) const { return sc_mass_2d(static_cast<T>(alpha), R); }
+    __device__ T green_mass(T R) const {
+        const T a = static_cast<T>(alpha);
+        return sc_mass_2d(a, sc_ball_2d(a, R));
+    }
     template <typename T, class Rng>
     __device__ T green_radius(T R, Rng &rng, bool &overflow) const {
-        return sc_sample_radius_2d(static_cast<T>(alpha), R, rng, overflow);
+        const T a = static_cast<T>(alpha);
+        return sc_sample_radius_2d(a, sc_ball_2d(a, R), rng, overflow);
     }
     template <typename T>
     __device__ T screening(T R) const { return sc_weight_2d(static_cast<T>(alpha), R); }
@@ -708,12 +880,32 @@ __device__ __forceinline__ double mis_contribution(const Eq &eq, V3<T> p, T R, R
     return source_value == 0.0 ? 0.0 : green_value * source_value / mixture_pdf;
 }
 
-// One iteration of the walk loop body before the closest-point query
-// (include/wos/wos.hpp:69-115): the source contribution of the current ball,
-// the screening weight, then the step to the sphere.  Returns the new point.
+// Equations whose source and weight share a ScreenedBall (kBalls), and whose
+// Green radius is drawn by rejection.
+template <class Eq, class = void>
+struct HasBalls {
+    static constexpr bool value = false;
+};
+template <class Eq>
+struct HasBalls<Eq, decltype(void(Eq::kBalls))> {
+    static constexpr bool value = Eq::kBalls;
+};
+
+// The source sample at an accepted Green radius.
+template <int DIM, bool EXACT, typename T, class Eq, class Rng>
+__device__ __forceinline__ void add_ball_source(const Eq &eq, V3<T> p, const ScreenedBall<T> &b,
+                                                T radius, T &sample, T weight, Rng &src) {
+    const V3<T> sp = direction_at<DIM, EXACT, T>(p, radius, src);
+    const T f = eq.source(sp);
+    if (f != T(0)) sample += weight * sc_mass_2d(static_cast<T>(eq.alpha), b) * f;
+}
+
+// The walk loop body but for the Green samples of kBalls equations, which
+// walk_body and the walk kernels' proposal loop draw.
 template <int DIM, bool EXACT, typename T, class Eq, class WalkRng, class SrcRng>
-__device__ __forceinline__ V3<T> walk_body(const Eq &eq, V3<T> p, T R, T &sample, T &weight,
-                                           WalkRng &walk, SrcRng &src, bool &overflow) {
+__device__ __forceinline__ V3<T> walk_body_direct(const Eq &eq, V3<T> p, T R, T &sample,
+                                                  T &weight, WalkRng &walk, SrcRng &src,
+                                                  bool &overflow) {
     if constexpr (Eq::kSource) {
         bool may = true;
         if (DIM == 2) may = eq.may_intersect(p, R);
@@ -726,7 +918,7 @@ __device__ __forceinline__ V3<T> walk_body(const Eq &eq, V3<T> p, T R, T &sample
             }
         }
         if (may && !mis) {
-            if (eq.mode == kGreen) {
+            if (!HasBalls<Eq>::value && eq.mode == kGreen) {
                 const T radius = eq.green_radius(R, src, overflow);
                 const V3<T> sp = direction_at<DIM, EXACT, T>(p, radius, src);
                 const T f = eq.source(sp);
@@ -742,6 +934,25 @@ __device__ __forceinline__ V3<T> walk_body(const Eq &eq, V3<T> p, T R, T &sample
     }
     if constexpr (Eq::kScreening) weight *= eq.screening(R);
     return sphere_step<DIM, EXACT, T>(p, R, walk);
+}
+
+// One iteration of the walk loop body before the closest-point query
+// (include/wos/wos.hpp:69-115): the source contribution of the current ball,
+// the screening weight, then the step to the sphere.  Returns the new point.
+template <int DIM, bool EXACT, typename T, class Eq, class WalkRng, class SrcRng>
+__device__ __forceinline__ V3<T> walk_body(const Eq &eq, V3<T> p, T R, T &sample, T &weight,
+                                           WalkRng &walk, SrcRng &src, bool &overflow) {
+    if constexpr (HasBalls<Eq>::value) {
+        if (eq.mode == kGreen && eq.may_intersect(p, R)) {
+            const T a = static_cast<T>(eq.alpha);
+            const ScreenedBall<T> b = sc_ball_2d(a, R);
+            const T radius = sc_sample_radius_2d(a, b, src, overflow);
+            add_ball_source<DIM, EXACT, T>(eq, p, b, radius, sample, weight, src);
+            weight *= sc_weight_2d(b);
+            return sphere_step<DIM, EXACT, T>(p, R, walk);
+        }
+    }
+    return walk_body_direct<DIM, EXACT, T>(eq, p, R, sample, weight, walk, src, overflow);
 }
 
 }  // namespace wosb

@@ -137,43 +137,62 @@ __device__ __forceinline__ float as_i0_small(float x) {  // 9.8.1, |x| < 3.75
                      u * (1.2067492f + u * (0.2659732f + u * (0.0360768f + u * 0.0045813f)))));
 }
 
+__device__ __forceinline__ float as_i0_large(float u) {  // 9.8.2, u = 3.75 / x
+    return 0.39894228f +
+           u * (0.01328592f +
+                u * (0.00225319f +
+                     u * (-0.00157565f +
+                          u * (0.00916281f +
+                               u * (-0.02057706f +
+                                    u * (0.02635537f +
+                                         u * (-0.01647633f + u * 0.00392377f)))))));
+}
+__device__ __forceinline__ float as_k0_rest(float y) {  // 9.8.5, K0 + ln(x/2) I0, y = x^2 / 4
+    return -0.57721566f +
+           y * (0.42278420f +
+                y * (0.23069756f +
+                     y * (0.03488590f + y * (0.00262698f + y * (0.00010750f + y * 0.0000074f)))));
+}
+__device__ __forceinline__ float as_k0_large(float u) {  // 9.8.6, u = 2 / x
+    return 1.25331414f +
+           u * (-0.07832358f +
+                u * (0.02189568f +
+                     u * (-0.01062446f + u * (0.00587872f + u * (-0.00251540f + u * 0.00053208f)))));
+}
+
 template <>
 __device__ __forceinline__ float log_i0<float>(float x) {
     x = fabsf(x);
     if (x < 3.75f) return logf(as_i0_small(x));
-    const float u = 3.75f / x;  // 9.8.2
-    const float q =
-        0.39894228f +
-        u * (0.01328592f +
-             u * (0.00225319f +
-                  u * (-0.00157565f +
-                       u * (0.00916281f +
-                            u * (-0.02057706f +
-                                 u * (0.02635537f + u * (-0.01647633f + u * 0.00392377f)))))));
-    return x - 0.5f * logf(x) + logf(q);
+    return x - 0.5f * logf(x) + logf(as_i0_large(3.75f / x));
 }
 
 template <>
 __device__ __forceinline__ float log_k0<float>(float x) {
     if (x < 0.0f) return NAN;
     if (x == 0.0f) return INFINITY;
-    if (x <= 2.0f) {  // 9.8.5
+    if (x <= 2.0f) {
         const float y = 0.25f * x * x;
-        const float k =
-            -logf(0.5f * x) * as_i0_small(x) +
-            (-0.57721566f +
-             y * (0.42278420f +
-                  y * (0.23069756f +
-                       y * (0.03488590f + y * (0.00262698f + y * (0.00010750f + y * 0.0000074f))))));
+        const float k = -logf(0.5f * x) * as_i0_small(x) + as_k0_rest(y);
         return logf(k);
     }
-    const float u = 2.0f / x;  // 9.8.6
-    const float q =
-        1.25331414f +
-        u * (-0.07832358f +
-             u * (0.02189568f +
-                  u * (-0.01062446f + u * (0.00587872f + u * (-0.00251540f + u * 0.00053208f)))));
-    return -x - 0.5f * logf(x) + logf(q);
+    return -x - 0.5f * logf(x) + logf(as_k0_large(2.0f / x));
+}
+
+// The same approximants with the hardware's approximate logarithm, reciprocal
+// and root, for tests that settle a close call with the forms above: K0(x) for
+// 0 < x <= 2, ln I0(x) and ln K0(x) for x > 0, within about 1e-6 of K0 or
+// (1 + x) 1e-6 of the logarithms.
+__device__ __forceinline__ float quick_k0_small(float x, float i0) {
+    return as_k0_rest(0.25f * x * x) - __logf(0.5f * x) * i0;
+}
+__device__ __forceinline__ float quick_log_i0(float x) {
+    return x < 3.75f ? __logf(as_i0_small(x))
+                     : x + __logf(as_i0_large(__fdividef(3.75f, x)) * __frsqrt_rn(x));
+}
+__device__ __forceinline__ float quick_log_k0(float x) {
+    return x <= 2.0f ? __logf(quick_k0_small(x, as_i0_small(x)))
+                     : __logf(as_k0_large(__fdividef(2.0f, x)) * __frsqrt_rn(x)) - x;
 }
 
 // include/wos/fastmath.hpp:15-28 (series truncated at a 1e-8 term)

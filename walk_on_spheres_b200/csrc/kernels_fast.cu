@@ -74,15 +74,16 @@ __device__ __forceinline__ void write_partial(const FastArgs &a, unsigned long l
 // slots from kPool - 1 down walks to be resumed with the radius found.
 constexpr int kPool = 64;
 
-template <int DIM, class Eq>
+template <int DIM, class Eq, int HC>
 struct WalkPool {
     static constexpr int kFields = 5 + (DIM == 3) + (Eq::kSource ? 1 : 0) +
-                                   (Eq::kScreening ? 1 : 0);
+                                   (Eq::kScreening ? 1 : 0) + (HC == kLaneScan ? 1 : 0);
     unsigned *f;
     __device__ __forceinline__ float &real(int field, int i) {
         return reinterpret_cast<float *>(f)[field * kPool + i];
     }
     __device__ __forceinline__ float &radius(int i) { return real(4, i); }
+    __device__ __forceinline__ unsigned &slot(int i) { return f[(kFields - 1) * kPool + i]; }
     __device__ __forceinline__ void put(int i, V3<float> p, float sample, float weight, int steps,
                                         int walk) {
         f[i] = static_cast<unsigned>(steps);
@@ -108,14 +109,6 @@ struct WalkPool {
     }
 };
 
-// Which walk kernels put walks aside: FAST_FP32 ones, except on lane-scan
-// scenes, where a query is one short scan that every lane runs at every step.
-// Measured there against fast_task: laplace and poisson 3-4% faster with the
-// pool, screened_poisson 5% and the transient plate 11% slower (their
-// rejection samplers fill the step, and the pool costs registers).
-template <typename T, int HC>
-constexpr bool kPooled = std::is_same<T, float>::value && HC != kLaneScan;
-
 // One FAST_FP32 task: walks [c*chunk, min(N, (c+1)*chunk)) of point pidx,
 // written to a.partials[task].  The lanes only take steps; a walk whose step
 // needs a query (near the boundary: mostly its last step) is put aside in
@@ -135,7 +128,7 @@ __device__ __forceinline__ void fast_task32(const FastArgs a, const WideView &wv
                                             unsigned *s_pool) {
     const int lane = threadIdx.x & 31;
     const unsigned lt_mask = (1u << lane) - 1u;
-    WalkPool<DIM, Eq> pool{s_pool};
+    WalkPool<DIM, Eq, HC> pool{s_pool};
 
     double x0, y0, z0;
     uint64_t linear;
@@ -173,6 +166,15 @@ __device__ __forceinline__ void fast_task32(const FastArgs a, const WideView &wv
     int waiting = 0;  // walks waiting for a query
     int resume = 0;   // walks waiting for a lane
     const uint2 pkey = PhiloxStream::key_of(pseed);
+    FastRng<float> rng(pkey, 0u);
+    // kBalls equations with Green sampling: a step whose source radius is
+    // still being drawn keeps its lane.  An iteration makes one proposal, so
+    // lanes that accept go on while others try again (in a loop of its own
+    // the sampler ran until the last of 32 lanes had accepted)
+    bool trying = false;
+    ScreenedBall<float> ball{0.0f, 0.0f, 0.0f, 0.0f};
+    float green_r = 0.0f;
+    int tries = 0;
 
     for (;;) {
         // lanes without a walk take one: a resumed walk, else a new one
@@ -202,29 +204,78 @@ __device__ __forceinline__ void fast_task32(const FastArgs a, const WideView &wv
         }
         // one step of every walk in flight
         bool defer = false;
-        if (active) {
-            FastRng<float> rng(pkey, static_cast<uint32_t>(walk));
+        int near_slot = -1;  // lane-scan scenes: winner of the query
+        bool sampled = false;
+        if (active && !trying) {
+            rng = FastRng<float>(pkey, static_cast<uint32_t>(walk));
             rng.begin_step(steps);
-            p = walk_body<DIM, false, float>(eq, p, R, sample, weight, rng, rng, overflow);
+        }
+        if constexpr (HasBalls<Eq>::value) {
+            // (each part for the whole warp: a lane that accepts waits for
+            // the others here, not at the end of its step)
+            const float alpha = static_cast<float>(eq.alpha);
+            if (active && !trying && eq.mode == kGreen && eq.may_intersect(p, R)) {
+                ball = sc_ball_2d(alpha, R);
+                green_r = ball.R * 0.5f;
+                trying = true;
+                tries = 0;
+            }
+            __syncwarp();
+            if (trying) {
+                sampled = sc_try_radius_2d(alpha, ball, rng, green_r);
+                if (!sampled && ++tries == kRejectionCap) {
+                    overflow = true;
+                    sampled = true;
+                }
+                trying = !sampled;
+            }
+            __syncwarp();
+            if (sampled) {
+                add_ball_source<DIM, false, float>(eq, p, ball, green_r, sample, weight, rng);
+                weight *= sc_weight_2d(ball);
+                p = sphere_step<DIM, false, float>(p, R, rng);
+            }
+        }
+        const bool stepped = active && !trying;
+        if (stepped && !sampled) {
+            p = walk_body_direct<DIM, false, float>(eq, p, R, sample, weight, rng, rng, overflow);
+        }
+        if constexpr (HasBalls<Eq>::value) __syncwarp();
+        if (stepped) {
             ++steps;
-            defer = true;
-            // away from the shell a lattice lower bound is a valid (smaller)
-            // radius and spares the exact query; the step that reaches the
-            // cap queries, for its nearest point
-            if (wv.gd != nullptr && steps < a.max_steps) {
-                const LatticeSample ls = lattice_sample<DIM>(wv, p.x, p.y, DIM == 3 ? p.z : 0.0f);
-                const float gb = (ls.d - ls.r) * a.shrink;
-                if (ls.d >= wv.gratio * ls.r && gb > 0.0f && gb * gb > a.shell2) {
-                    R = gb;
-                    defer = false;
+            if constexpr (HC == kLaneScan) {
+                // a handful of primitives: every lane scans them for its own query
+                const WideResult q = lane_nearest<DIM>(wv, p.x, p.y, p.z);
+                const float r = sqrtf(q.best);
+                R = q.best > a.shell2 ? r * a.shrink : r;
+                near_slot = q.slot;
+                defer = R * R <= a.shell2 || steps >= a.max_steps;
+            } else {
+                defer = true;
+                // away from the shell a lattice lower bound is a valid
+                // (smaller) radius and spares the exact query; the step
+                // that reaches the cap queries, for its nearest point
+                if (wv.gd != nullptr && steps < a.max_steps) {
+                    const LatticeSample ls =
+                        lattice_sample<DIM>(wv, p.x, p.y, DIM == 3 ? p.z : 0.0f);
+                    const float gb = (ls.d - ls.r) * a.shrink;
+                    if (ls.d >= wv.gratio * ls.r && gb > 0.0f && gb * gb > a.shell2) {
+                        R = gb;
+                        defer = false;
+                    }
                 }
             }
         }
+        if constexpr (HC == kLaneScan) queries += __popc(__ballot_sync(kFull, stepped));
         const unsigned put = __ballot_sync(kFull, defer);
         if (put) {
             if (defer) {
                 const int i = waiting + __popc(put & lt_mask);
                 pool.put(i, p, sample, weight, steps, walk);
+                if constexpr (HC == kLaneScan) {
+                    pool.radius(i) = R;
+                    pool.slot(i) = static_cast<unsigned>(near_slot);
+                }
                 active = false;
             }
             waiting += __popc(put);
@@ -241,53 +292,62 @@ __device__ __forceinline__ void fast_task32(const FastArgs a, const WideView &wv
         V3<float> q{0.0f, 0.0f, 0.0f};
         float qR = 0.0f, qsample = 0.0f, qweight = 1.0f;
         int qsteps = 0, qwalk = 0, slot = -1;
-        int packed = -1;  // the node's candidate list, if any
-        if (has) {
-            pool.get(waiting + lane, q, qsample, qweight, qsteps, qwalk);
-            if (wv.gl != nullptr && qsteps < a.max_steps) {
-                const LatticeSample ls = lattice_sample<DIM>(wv, q.x, q.y, DIM == 3 ? q.z : 0.0f);
-                if (ls.d <= a.list_t) {
-                    const int2 e = __ldg(wv.gl + ls.node);
-                    packed = DIM == 3 && e.x >= 0 ? list_prefix(wv, e, ls.r) : e.x;
+        if constexpr (HC == kLaneScan) {
+            if (has) {
+                pool.get(waiting + lane, q, qsample, qweight, qsteps, qwalk);
+                qR = pool.radius(waiting + lane);
+                slot = static_cast<int>(pool.slot(waiting + lane));
+            }
+            __syncwarp();
+        } else {
+            int packed = -1;  // the node's candidate list, if any
+            if (has) {
+                pool.get(waiting + lane, q, qsample, qweight, qsteps, qwalk);
+                if (wv.gl != nullptr && qsteps < a.max_steps) {
+                    const LatticeSample ls = lattice_sample<DIM>(wv, q.x, q.y, DIM == 3 ? q.z : 0.0f);
+                    if (ls.d <= a.list_t) {
+                        const int2 e = __ldg(wv.gl + ls.node);
+                        packed = DIM == 3 && e.x >= 0 ? list_prefix(wv, e, ls.r) : e.x;
+                    }
                 }
             }
-        }
-        __syncwarp();
-        const bool want = has && packed >= 0;
-        float qbest = 0.0f;
-        if constexpr (DIM == 2) {
-            if (want) {
+            __syncwarp();
+            const bool want = has && packed >= 0;
+            float qbest = 0.0f;
+            if constexpr (DIM == 2) {
+                if (want) {
+                    const WideResult r =
+                        list_nearest<DIM>(wv, list_of(wv, packed), list_length(packed), q.x, q.y,
+                                          0.0f);
+                    qbest = r.best;
+                    slot = r.slot;
+                }
+            } else if (__any_sync(kFull, want)) {
                 const WideResult r =
-                    list_nearest<DIM>(wv, list_of(wv, packed), list_length(packed), q.x, q.y,
-                                      0.0f);
-                qbest = r.best;
-                slot = r.slot;
+                    warp_list_nearest<DIM>(wv, want, packed, q.x, q.y, q.z);
+                if (want) {
+                    qbest = r.best;
+                    slot = r.slot;
+                }
             }
-        } else if (__any_sync(kFull, want)) {
-            const WideResult r =
-                warp_list_nearest<DIM>(wv, want, packed, q.x, q.y, q.z);
-            if (want) {
-                qbest = r.best;
-                slot = r.slot;
+            // no list: the warp resolves each such query together
+            unsigned pending = __ballot_sync(kFull, has && packed < 0);
+            while (pending) {
+                const int j = __ffs(pending) - 1;
+                pending &= pending - 1u;
+                const float qx = __shfl_sync(kFull, q.x, j);
+                const float qy = __shfl_sync(kFull, q.y, j);
+                const float qz = DIM == 3 ? __shfl_sync(kFull, q.z, j) : 0.0f;
+                const WideResult r = wide_nearest<DIM, HC>(wv, qx, qy, qz, a.keep, a.exact2);
+                if (lane == j) {
+                    qbest = r.best;
+                    slot = r.slot;
+                }
             }
+            queries += m;
+            const float r = sqrtf(qbest);
+            qR = qbest > a.shell2 ? r * a.shrink : r;
         }
-        // no list: the warp resolves each such query together
-        unsigned pending = __ballot_sync(kFull, has && packed < 0);
-        while (pending) {
-            const int j = __ffs(pending) - 1;
-            pending &= pending - 1u;
-            const float qx = __shfl_sync(kFull, q.x, j);
-            const float qy = __shfl_sync(kFull, q.y, j);
-            const float qz = DIM == 3 ? __shfl_sync(kFull, q.z, j) : 0.0f;
-            const WideResult r = wide_nearest<DIM, HC>(wv, qx, qy, qz, a.keep, a.exact2);
-            if (lane == j) {
-                qbest = r.best;
-                slot = r.slot;
-            }
-        }
-        queries += m;
-        const float r = sqrtf(qbest);
-        qR = qbest > a.shell2 ? r * a.shrink : r;
         bool go_on = false;
         if (has) {
             bool stop = false;
@@ -343,25 +403,21 @@ __device__ __forceinline__ void fast_task32(const FastArgs a, const WideView &wv
     write_partial<true>(a, task, acc, steps_acc, hits, queries, overflow, bad);
 }
 
-// One task: walks [c*chunk, min(N, (c+1)*chunk)) of point pidx, written to
-// a.partials[task] as Welford statistics.
-template <int DIM, class Eq, typename T, int HC>
-__device__ __forceinline__ void fast_task(const FastArgs a, const WideView &wv, const Eq &eq,
-                                          unsigned long long task, long long pidx, int c) {
-    constexpr bool kF32 = std::is_same<T, float>::value;
+// One FAST_FP64 task: walks [c*chunk, min(N, (c+1)*chunk)) of point pidx, each
+// lane regenerated with the next walk when its walk ends.
+template <int DIM, class Eq>
+__device__ __forceinline__ void fast_task64(const FastArgs a, const WideView &wv, const Eq &eq,
+                                            unsigned long long task, long long pidx, int c) {
     const int lane = threadIdx.x & 31;
     const unsigned lt_mask = (1u << lane) - 1u;
     const double eps = a.eps;
-    const double eps2 = eps * eps;
 
-    double x0, y0, z0;
+    V3<double> p0;
     uint64_t linear;
-    point_at(a.ps, pidx, x0, y0, z0, linear);
+    point_at(a.ps, pidx, p0.x, p0.y, p0.z, linear);
     const uint64_t pseed = point_seed(a.seed, linear);
-    const V3<T> p0{static_cast<T>(x0), static_cast<T>(y0), static_cast<T>(z0)};
-    const double r0 = a.start[pidx].radius;
-    const T R0 = static_cast<T>(r0);
-    const bool start_stops = !(r0 > eps);  // start point already inside the shell
+    const double R0 = a.start[pidx].radius;
+    const bool start_stops = !(R0 > eps);  // start point already inside the shell
     const int w0 = c * a.chunk;
     const int w1 = min(a.n_walks, w0 + a.chunk);
 
@@ -369,218 +425,70 @@ __device__ __forceinline__ void fast_task(const FastArgs a, const WideView &wv, 
     int steps_acc = 0;
     ShiftedSums acc;
     unsigned hits = 0;
-    // BVH closest-point queries of this task (warp-uniform; FP32 only: every
-    // FP64 step is one).  At most chunk * max_steps < 2^32 (set_chunk).
-    unsigned queries = 0;
     bool overflow = false;
-    bool bad = false;  // a closest-point query found no primitive
 
     // per-lane walk state
     int walk = w0 + lane;
     bool active = walk < w1;
     int next = w0 + 32;
-    V3<T> p = p0;
-    T R = R0;
-    T sample = T(0), weight = T(1);
+    V3<double> p = p0;
+    double R = R0;
+    double sample = 0.0, weight = 1.0;
     int steps = 0;
-    int slot = -1;                 // winner of the last query (FP32: wide slot, FP64: binary)
-    V3<double> np64{0.0, 0.0, 0.0};  // FP64: nearest point of the last query
-    int bid64 = -1;
+    V3<double> np{0.0, 0.0, 0.0};  // nearest point of the last query
+    int bid = -1;
     const uint2 pkey = PhiloxStream::key_of(pseed);
-    FastRng<T> rng(pkey, static_cast<uint32_t>(walk));
+    FastRng<double> rng(pkey, static_cast<uint32_t>(walk));
 
     while (__any_sync(kFull, active)) {
-        bool need_query = false;
-        bool listed = false;  // answered from a near-boundary list
-        int packed = -1;      // 3D: the list the warp scans for this lane
         // One step of every walk in flight (a start point inside the shell
         // takes none: its walks end where they start).
-        if (active && !start_stops) {
+        const bool query = active && !start_stops;
+        if (query) {
             rng.begin_step(steps);
-            p = walk_body<DIM, false, T>(eq, p, R, sample, weight, rng, rng, overflow);
+            p = walk_body<DIM, false, double>(eq, p, R, sample, weight, rng, rng, overflow);
             ++steps;
-            if constexpr (kF32) {
-                need_query = true;
-                if constexpr (HC != kLaneScan) {
-                    // away from the shell a lattice lower bound is a valid
-                    // (smaller) radius and spares the exact query; the step
-                    // that reaches the cap queries, for its nearest point
-                    if (wv.gd != nullptr && steps < a.max_steps) {
-                        const LatticeSample ls =
-                            lattice_sample<DIM>(wv, p.x, p.y, DIM == 3 ? p.z : 0.0f);
-                        const float gb = (ls.d - ls.r) * a.shrink;
-                        if (ls.d >= wv.gratio * ls.r && gb > 0.0f && gb * gb > a.shell2) {
-                            R = gb;
-                            need_query = false;
-                        } else if (ls.d <= a.list_t) {
-                            // near the boundary: a query over the node's
-                            // candidate list, when it has one; in 2D (a
-                            // few segments) this lane scans it, in 3D the
-                            // warp scans all such lists together below
-                            const int2 e = __ldg(wv.gl + ls.node);
-                            const int v = DIM == 3 && e.x >= 0 ? list_prefix(wv, e, ls.r) : e.x;
-                            if (v >= 0) {
-                                if constexpr (DIM == 2) {
-                                    const WideResult q = list_nearest<DIM>(
-                                        wv, list_of(wv, v), list_length(v),
-                                        static_cast<float>(p.x), static_cast<float>(p.y), 0.0f);
-                                    const float r = sqrtf(q.best);
-                                    R = static_cast<T>(q.best > a.shell2 ? r * a.shrink : r);
-                                    slot = q.slot;
-                                } else {
-                                    packed = v;
-                                }
-                                need_query = false;
-                                listed = true;
-                            }
-                        }
-                    }
-                }
-            } else {
-                need_query = true;
-            }
         }
-        if constexpr (!kF32) {
-            // FP64 queries by the whole warp, one lane's after another; the
+        if (wv.margin64 >= 0.0f && wv.n > thread_query_prims(DIM)) {
+            // queries by the whole warp, one lane's after another; the
             // winners' distances then for all lanes at once
-            if (wv.margin64 >= 0.0f && wv.n > thread_query_prims(DIM)) {
-                Candidates cand{0, -1};
-                unsigned pending = __ballot_sync(kFull, need_query);
-                while (pending) {
-                    const int j = __ffs(pending) - 1;
-                    pending &= pending - 1u;
-                    const double qx = __shfl_sync(kFull, static_cast<double>(p.x), j);
-                    const double qy = __shfl_sync(kFull, static_cast<double>(p.y), j);
-                    const double qz =
-                        DIM == 3 ? __shfl_sync(kFull, static_cast<double>(p.z), j) : 0.0;
-                    const Candidates c = warp_candidates64<DIM>(a.s, wv, qx, qy, qz);
-                    if (lane == j) cand = c;
-                }
-                if (need_query) {
-                    R = static_cast<T>(sqrt(pick_nearest64<DIM>(
-                        a.s, cand, static_cast<double>(p.x), static_cast<double>(p.y),
-                        static_cast<double>(p.z), slot, np64.x, np64.y, np64.z)));
-                    bid64 = bid_of<DIM>(a.s, slot);
-                }
-            } else if (need_query) {
-                const Nearest<double> q = nearest64<DIM>(
-                    a.s, static_cast<double>(p.x), static_cast<double>(p.y),
-                    static_cast<double>(p.z), dinf());
-                R = static_cast<T>(sqrt(q.best));
-                np64 = V3<double>{q.x, q.y, q.z};
-                bid64 = bid_of<DIM>(a.s, q.slot);
-            }
-        }
-        if constexpr (kF32 && HC == kLaneScan) {
-            // a handful of primitives: every lane scans them for its own query
-            queries += __popc(__ballot_sync(kFull, need_query));
-            if (need_query) {
-                const WideResult q = lane_nearest<DIM>(wv, static_cast<float>(p.x),
-                                                       static_cast<float>(p.y),
-                                                       static_cast<float>(p.z));
-                const float r = sqrtf(q.best);
-                R = static_cast<T>(q.best > a.shell2 ? r * a.shrink : r);
-                slot = q.slot;
-            }
-        } else if constexpr (kF32) {
-            if constexpr (DIM == 3) {
-                const bool want = packed >= 0;
-                if (__any_sync(kFull, want)) {
-                    const WideResult q = warp_list_nearest<DIM>(
-                        wv, want, packed, static_cast<float>(p.x), static_cast<float>(p.y),
-                        static_cast<float>(p.z));
-                    if (want) {
-                        const float r = sqrtf(q.best);
-                        R = static_cast<T>(q.best > a.shell2 ? r * a.shrink : r);
-                        slot = q.slot;
-                    }
-                }
-            }
-            // the warp resolves every pending closest-point query together
-            unsigned pending = __ballot_sync(kFull, need_query);
-            queries += __popc(pending) + __popc(__ballot_sync(kFull, listed));
-            float qbest = 0.0f;
-            int qslot = -1;
+            Candidates cand{0, -1};
+            unsigned pending = __ballot_sync(kFull, query);
             while (pending) {
                 const int j = __ffs(pending) - 1;
                 pending &= pending - 1u;
-                const float qx = __shfl_sync(kFull, static_cast<float>(p.x), j);
-                const float qy = __shfl_sync(kFull, static_cast<float>(p.y), j);
-                const float qz = DIM == 3 ? __shfl_sync(kFull, static_cast<float>(p.z), j) : 0.0f;
-                const WideResult r = wide_nearest<DIM, HC>(wv, qx, qy, qz, a.keep, a.exact2);
-                if (lane == j) {
-                    qbest = r.best;
-                    qslot = r.slot;
-                }
+                const double qx = __shfl_sync(kFull, p.x, j);
+                const double qy = __shfl_sync(kFull, p.y, j);
+                const double qz = DIM == 3 ? __shfl_sync(kFull, p.z, j) : 0.0;
+                const Candidates found = warp_candidates64<DIM>(a.s, wv, qx, qy, qz);
+                if (lane == j) cand = found;
             }
-            if (need_query) {
-                const float r = sqrtf(qbest);
-                R = static_cast<T>(qbest > a.shell2 ? r * a.shrink : r);
-                slot = qslot;
+            if (query) {
+                int slot;
+                R = sqrt(pick_nearest64<DIM>(a.s, cand, p.x, p.y, p.z, slot, np.x, np.y, np.z));
+                bid = bid_of<DIM>(a.s, slot);
             }
+        } else if (query) {
+            const Nearest<double> q = nearest64<DIM>(a.s, p.x, p.y, p.z, dinf());
+            R = sqrt(q.best);
+            np = V3<double>{q.x, q.y, q.z};
+            bid = bid_of<DIM>(a.s, q.slot);
         }
         // Walks whose new radius is in the epsilon shell, or that reached
-        // the step cap, end in the iteration of their last step, so the lane
-        // steps its next walk in the next iteration.
-        bool done = false;
-        double value = 0.0;
-        if (active) {
-            bool stop = false;
-            V3<double> np{0.0, 0.0, 0.0};
-            int bid = -1;
+        // the step cap (include/wos/wos.hpp:129-137), end in the iteration of
+        // their last step, so the lane steps its next walk in the next one.
+        bool done = active && (start_stops || !(R > eps));
+        if (active && !done && steps >= a.max_steps) {
+            ++hits;
+            done = true;
+        }
+        if (done) {
             if (start_stops) {
-                stop = true;
                 const StartRecord st = a.start[pidx];
                 np = V3<double>{st.nx, st.ny, st.nz};
                 bid = st.boundary_id;
-            } else if (!kF32) {
-                stop = !(static_cast<double>(R) > eps);
-                np = np64;
-                bid = bid64;
-            } else if (static_cast<float>(R) * static_cast<float>(R) <= a.shell2) {
-                // epsilon shell: FP64 re-projection onto the nearest primitive
-                // (a query that found none is a broken walk: flag it, stop)
-                if (slot < 0) {
-                    bad = true;
-                    stop = true;
-                } else {
-                    const double d2 = reproject64_sq<DIM>(a.s, wv.wide2bin[slot],
-                                                          static_cast<double>(p.x),
-                                                          static_cast<double>(p.y),
-                                                          static_cast<double>(p.z), np, bid);
-                    if (d2 <= eps2) {
-                        stop = true;
-                    } else {
-                        R = static_cast<T>(sqrt(d2));
-                    }
-                }
             }
-            if (!stop && steps >= a.max_steps) {
-                // step cap: finish at the nearest boundary point
-                // (include/wos/wos.hpp:129-137)
-                ++hits;
-                stop = true;
-                if (kF32) {
-                    if (slot < 0) {
-                        bad = true;
-                    } else {
-                        reproject64<DIM>(a.s, wv.wide2bin[slot], static_cast<double>(p.x),
-                                         static_cast<double>(p.y), static_cast<double>(p.z), np,
-                                         bid);
-                    }
-                } else {
-                    np = np64;
-                    bid = bid64;
-                }
-            }
-            if (stop) {
-                value = static_cast<double>(sample) +
-                        static_cast<double>(weight) * eq.boundary(np, bid);
-                done = true;
-            }
-        }
-        if (done) {
-            acc.add(value);
+            acc.add(sample + weight * eq.boundary(np, bid));
             steps_acc += steps;
         }
         const unsigned done_mask = __ballot_sync(kFull, done);
@@ -591,17 +499,25 @@ __device__ __forceinline__ void fast_task(const FastArgs a, const WideView &wv, 
                 if (active) {
                     p = p0;
                     R = R0;
-                    sample = T(0);
-                    weight = T(1);
+                    sample = 0.0;
+                    weight = 1.0;
                     steps = 0;
-                    rng = FastRng<T>(pkey, static_cast<uint32_t>(walk));
+                    rng = FastRng<double>(pkey, static_cast<uint32_t>(walk));
                 }
             }
             next += __popc(done_mask);
         }
     }
+    write_partial<false>(a, task, acc, steps_acc, hits, 0u, overflow, false);
+}
 
-    write_partial<kF32>(a, task, acc, steps_acc, hits, queries, overflow, bad);
+// Blocks per SM of the FP32 walk kernels: 4 (64 registers) for the height <= 3
+// traversals (5 spill: disk 7.2 -> 8.6 ms); 3 for the generic and lane-scan
+// ones and for equations with a rejection sampler, whose state would spill
+// (star of 777 segments, screened, Green: 3.89 -> 3.78 ms, uniform 2.65 -> 2.35).
+template <class Eq, int HC>
+constexpr int min_blocks32() {
+    return (HC == kHeightUpTo2 || HC == kHeight3) && !HasBalls<Eq>::value ? 4 : 3;
 }
 
 // Blocks per SM of the FP64 walk kernels (80 / 128 registers at 3 / 2): their
@@ -634,8 +550,7 @@ __global__ void __launch_bounds__(256, MIN_BLOCKS) walk_fast_kernel(FastArgs a, 
     constexpr bool kF32 = std::is_same<T, float>::value;
     extern __shared__ float4 smem[];
     __shared__ int s_off[8];
-    __shared__ unsigned s_pool[kPooled<T, HC> ? 8 : 1]
-                              [kPooled<T, HC> ? WalkPool<DIM, Eq>::kFields * kPool : 1];
+    __shared__ unsigned s_pool[kF32 ? 8 : 1][kF32 ? WalkPool<DIM, Eq, HC>::kFields * kPool : 1];
     if (threadIdx.x < 8) s_off[threadIdx.x] = a.w.off[threadIdx.x];
     WideView wv = a.w;
     wv.off = s_off;
@@ -664,10 +579,10 @@ __global__ void __launch_bounds__(256, MIN_BLOCKS) walk_fast_kernel(FastArgs a, 
         const long long pidx = static_cast<long long>(task / a.chunks);
         const int c = static_cast<int>(task % a.chunks);
         if (a.location[pidx] != 1) continue;
-        if constexpr (kPooled<T, HC>) {
+        if constexpr (kF32) {
             fast_task32<DIM, Eq, HC>(a, wv, eq, task, pidx, c, s_pool[threadIdx.x >> 5]);
         } else {
-            fast_task<DIM, Eq, T, HC>(a, wv, eq, task, pidx, c);
+            fast_task64<DIM, Eq>(a, wv, eq, task, pidx, c);
         }
     }
 }
@@ -680,9 +595,9 @@ template <int DIM, class Eq, typename T, int MIN_BLOCKS, int HC>
 __global__ void __launch_bounds__(256, MIN_BLOCKS)
     walk_batch_kernel(const BatchItem *__restrict__ items, int n_items, long long n_tasks,
                       unsigned long long *queue) {
+    constexpr bool kF32 = std::is_same<T, float>::value;
     __shared__ int s_off[8][8];  // per warp: wide-tree offsets of the warp's current item
-    __shared__ unsigned s_pool[kPooled<T, HC> ? 8 : 1]
-                              [kPooled<T, HC> ? WalkPool<DIM, Eq>::kFields * kPool : 1];
+    __shared__ unsigned s_pool[kF32 ? 8 : 1][kF32 ? WalkPool<DIM, Eq, HC>::kFields * kPool : 1];
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
     int cur = -1;
@@ -712,12 +627,11 @@ __global__ void __launch_bounds__(256, MIN_BLOCKS)
         WideView wv = it.a.w;
         wv.off = s_off[warp];
         const Eq eq = eq_from(it.eq, static_cast<Eq *>(nullptr));
-        if constexpr (kPooled<T, HC>) {
+        if constexpr (kF32) {
             fast_task32<DIM, Eq, HC>(it.a, wv, eq, static_cast<unsigned long long>(local), pidx, c,
                                      s_pool[warp]);
         } else {
-            fast_task<DIM, Eq, T, HC>(it.a, wv, eq, static_cast<unsigned long long>(local), pidx,
-                                      c);
+            fast_task64<DIM, Eq>(it.a, wv, eq, static_cast<unsigned long long>(local), pidx, c);
         }
     }
 }
@@ -785,7 +699,7 @@ cudaError_t batch_typed(int precision, int hc, const BatchItem *items, int n_ite
     if (precision == 32) {
         return with_height_class(hc, [&](auto h) {
             constexpr int HC = decltype(h)::value;
-            constexpr int kMinBlocks = (HC == kHeightUpTo2 || HC == kHeight3) ? 4 : 3;
+            constexpr int kMinBlocks = min_blocks32<Eq, HC>();
             walk_batch_kernel<DIM, Eq, float, kMinBlocks, HC><<<blocks, 256, 0, stream>>>(
                 items, n_items, n_tasks, queue);
             return cudaGetLastError();
@@ -803,7 +717,7 @@ cudaError_t batch_blocks_typed(int precision, int hc, int &blocks) {
     if (precision == 32) {
         e = with_height_class(hc, [&](auto h) {
             constexpr int HC = decltype(h)::value;
-            constexpr int kMinBlocks = (HC == kHeightUpTo2 || HC == kHeight3) ? 4 : 3;
+            constexpr int kMinBlocks = min_blocks32<Eq, HC>();
             return cudaOccupancyMaxActiveBlocksPerMultiprocessor(
                 &per_sm, walk_batch_kernel<DIM, Eq, float, kMinBlocks, HC>, 256, 0);
         });
@@ -937,9 +851,7 @@ cudaError_t launch_fast_typed(const FastArgs &a, const EqDesc &e, int precision,
     if (precision == 32) {
         return with_height_class(traversal_class(a.w), [&](auto h) -> cudaError_t {
             constexpr int HC = decltype(h)::value;
-            // 4 blocks / SM (64 registers) for the height <= 3 traversals,
-            // 3 for the generic one
-            constexpr int kMinBlocks = (HC == kHeightUpTo2 || HC == kHeight3) ? 4 : 3;
+            constexpr int kMinBlocks = min_blocks32<Eq, HC>();
             auto k = walk_fast_kernel<DIM, Eq, float, kMinBlocks, HC>;
             // (the walk pools are static shared memory beside it)
             if (plan.smem_bytes > 0) {

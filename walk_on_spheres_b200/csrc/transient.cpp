@@ -259,6 +259,7 @@ extern "C" int wos_transient_solve(wos_context *ctx, const wos_transient_params 
         t.ymin = ymin;
         t.ymax = ymax;
         t.cubic = p.cubic ? 1 : 0;
+        set_quotients(t);
     }
     WOS_CUDA(ctx, cudaMemcpyAsync(descs, host.data(), sizeof(TransientDesc) * steps,
                                   cudaMemcpyHostToDevice, stream),
