@@ -109,6 +109,45 @@ struct WalkPool {
     }
 };
 
+// A lane's statistics of the task at hand (ShiftedSums and the step count), in
+// shared memory behind the pool: they are touched once per 32 finished walks
+// and would hold nine registers through the steps.
+template <int OFFSET>
+struct LaneSums {
+    static constexpr int kWords = 8 * 32;
+    unsigned *f;
+    __device__ __forceinline__ double &real(int k, int lane) {
+        return reinterpret_cast<double *>(f + OFFSET)[k * 32 + lane];
+    }
+    __device__ __forceinline__ int &whole(int k, int lane) {
+        return reinterpret_cast<int *>(f + OFFSET + 6 * 32)[k * 32 + lane];
+    }
+    __device__ __forceinline__ void clear(int lane) {
+        whole(0, lane) = 0;
+        whole(1, lane) = 0;
+    }
+    __device__ __forceinline__ ShiftedSums values(int lane) {
+        ShiftedSums v;
+        v.n = whole(0, lane);
+        if (v.n > 0) {
+            v.k = real(0, lane);
+            v.s = real(1, lane);
+            v.q = real(2, lane);
+        }
+        return v;
+    }
+    __device__ __forceinline__ int steps(int lane) { return whole(1, lane); }
+    __device__ __forceinline__ void add(int lane, double value, int steps) {
+        ShiftedSums v = values(lane);
+        if (v.n == 0) real(0, lane) = value;
+        v.add(value);
+        whole(0, lane) = v.n;
+        real(1, lane) = v.s;
+        real(2, lane) = v.q;
+        whole(1, lane) += steps;
+    }
+};
+
 // One FAST_FP32 task: walks [c*chunk, min(N, (c+1)*chunk)) of point pidx,
 // written to a.partials[task].  The lanes only take steps; a walk whose step
 // needs a query (near the boundary: mostly its last step) is put aside in
@@ -140,8 +179,8 @@ __device__ __forceinline__ void fast_task32(const FastArgs a, const WideView &wv
     const int w0 = c * a.chunk;
     const int w1 = min(a.n_walks, w0 + a.chunk);
 
-    int steps_acc = 0;
-    ShiftedSums acc;
+    LaneSums<WalkPool<DIM, Eq, HC>::kFields * kPool> sums{s_pool};
+    sums.clear(lane);
     unsigned hits = 0;
     // BVH closest-point queries of this task (warp-uniform).  At most
     // chunk * max_steps < 2^32 (set_chunk).
@@ -153,8 +192,8 @@ __device__ __forceinline__ void fast_task32(const FastArgs a, const WideView &wv
         // the start point is inside the shell: every walk ends there
         const StartRecord st = a.start[pidx];
         const double value = eq.boundary(V3<double>{st.nx, st.ny, st.nz}, st.boundary_id);
-        for (int w = w0 + lane; w < w1; w += 32) acc.add(value);
-        write_partial<true>(a, task, acc, 0, 0u, 0u, false, false);
+        for (int w = w0 + lane; w < w1; w += 32) sums.add(lane, value, 0);
+        write_partial<true>(a, task, sums.values(lane), sums.steps(lane), 0u, 0u, false, false);
         return;
     }
 
@@ -383,9 +422,10 @@ __device__ __forceinline__ void fast_task32(const FastArgs a, const WideView &wv
                 }
             }
             if (stop) {
-                acc.add(static_cast<double>(qsample) +
-                        static_cast<double>(qweight) * eq.boundary(np, bid));
-                steps_acc += qsteps;
+                sums.add(lane,
+                         static_cast<double>(qsample) +
+                             static_cast<double>(qweight) * eq.boundary(np, bid),
+                         qsteps);
             }
             go_on = !stop;
         }
@@ -400,7 +440,8 @@ __device__ __forceinline__ void fast_task32(const FastArgs a, const WideView &wv
             __syncwarp();
         }
     }
-    write_partial<true>(a, task, acc, steps_acc, hits, queries, overflow, bad);
+    write_partial<true>(a, task, sums.values(lane), sums.steps(lane), hits, queries, overflow,
+                        bad);
 }
 
 // One FAST_FP64 task: walks [c*chunk, min(N, (c+1)*chunk)) of point pidx, each
@@ -511,6 +552,12 @@ __device__ __forceinline__ void fast_task64(const FastArgs a, const WideView &wv
     write_partial<false>(a, task, acc, steps_acc, hits, 0u, overflow, false);
 }
 
+// Shared memory of one warp's FP32 task: the pool and the lanes' sums.
+template <int DIM, class Eq, int HC>
+constexpr int pool_words() {
+    return WalkPool<DIM, Eq, HC>::kFields * kPool + 8 * 32;
+}
+
 // Blocks per SM of the FP32 walk kernels: 4 (64 registers) for the height <= 3
 // traversals (5 spill: disk 7.2 -> 8.6 ms); 3 for the generic and lane-scan
 // ones and for equations with a rejection sampler, whose state would spill
@@ -550,7 +597,7 @@ __global__ void __launch_bounds__(256, MIN_BLOCKS) walk_fast_kernel(FastArgs a, 
     constexpr bool kF32 = std::is_same<T, float>::value;
     extern __shared__ float4 smem[];
     __shared__ int s_off[8];
-    __shared__ unsigned s_pool[kF32 ? 8 : 1][kF32 ? WalkPool<DIM, Eq, HC>::kFields * kPool : 1];
+    __shared__ __align__(16) unsigned s_pool[kF32 ? 8 : 1][kF32 ? pool_words<DIM, Eq, HC>() : 4];
     if (threadIdx.x < 8) s_off[threadIdx.x] = a.w.off[threadIdx.x];
     WideView wv = a.w;
     wv.off = s_off;
@@ -597,7 +644,7 @@ __global__ void __launch_bounds__(256, MIN_BLOCKS)
                       unsigned long long *queue) {
     constexpr bool kF32 = std::is_same<T, float>::value;
     __shared__ int s_off[8][8];  // per warp: wide-tree offsets of the warp's current item
-    __shared__ unsigned s_pool[kF32 ? 8 : 1][kF32 ? WalkPool<DIM, Eq, HC>::kFields * kPool : 1];
+    __shared__ __align__(16) unsigned s_pool[kF32 ? 8 : 1][kF32 ? pool_words<DIM, Eq, HC>() : 4];
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
     int cur = -1;
@@ -1659,19 +1706,28 @@ FastPlan plan_fast(const SceneView &s, const WideView &w, long long n_points, in
             break;
         }
     }
+    // A solve that leaves warps without a task is over when its longest task
+    // is: shorter tasks then, down to one walk per lane (48 points x 256
+    // walks: 78 us at 256, 55 at 64, 49 at 32, 47 at 16).
+    while (chunk > 32 && n_points * ((n_walks + chunk - 1) / chunk) < warps) chunk /= 2;
     p.chunk = n_walks < chunk ? n_walks : chunk;
     if (p.chunk < 1) p.chunk = 1;
     p.chunks = (n_walks + p.chunk - 1) / p.chunk;
     p.n_tasks = n_points * p.chunks;
-    // stage the wide boxes, and the primitives too when they fit, in shared memory
-    const size_t box_floats = static_cast<size_t>(w.box_total);
-    const size_t prim_floats = static_cast<size_t>(w.dim == 2 ? 5 : 16) * w.npad;
+    // Stage the wide boxes, and the primitives too when they fit, in shared
+    // memory.  With near-boundary lists the tree is hardly read, so only a
+    // scene that costs no resident block is staged, and whole (disk of 1024
+    // segments, 21.5 KB: 7.10 ms staged, 7.25 not; star of 3000, 71 KB: 1.40
+    // and 0.99; blob of 60k triangles, boxes alone 84 KB: 4.29 and 3.30).
+    const size_t box_bytes = 4 * static_cast<size_t>(w.box_total);
+    const size_t prim_bytes = 4 * static_cast<size_t>(w.dim == 2 ? 5 : 16) * w.npad;
     const size_t cap = std::min<size_t>(96 * 1024, smem_optin);
-    p.stage_scene = precision == 32 && box_floats * 4 <= cap;
-    p.stage_prims = p.stage_scene && (box_floats + prim_floats) * 4 <= cap;
-    p.smem_bytes = p.stage_scene
-                       ? static_cast<int>((box_floats + (p.stage_prims ? prim_floats : 0)) * 4)
-                       : 0;
+    const bool lists = w.gl != nullptr;
+    p.stage_scene = precision == 32 &&
+                    (lists ? box_bytes + prim_bytes <= 24 * 1024 : box_bytes <= cap);
+    p.stage_prims = p.stage_scene && box_bytes + prim_bytes <= cap;
+    p.smem_bytes =
+        p.stage_scene ? static_cast<int>(box_bytes + (p.stage_prims ? prim_bytes : 0)) : 0;
     p.blocks = 0;  // sized from the occupancy of the chosen kernel at launch
     return p;
 }
