@@ -209,34 +209,552 @@ __device__ __forceinline__ double heat_source(const HeatArgs &a, V3<T> p, T R, F
     return mf;
 }
 
-template <int DIM, typename T, int MIN_BLOCKS, int HC>
-__global__ void __launch_bounds__(256, MIN_BLOCKS) heat_walk_kernel(HeatArgs a) {
-    constexpr bool kF32 = std::is_same<T, float>::value;
-    extern __shared__ float4 smem[];
-    __shared__ int s_off[8];
-    __shared__ double s_acc[10][256];
-    if (threadIdx.x < 8) s_off[threadIdx.x] = a.w.off[threadIdx.x];
-    WideView wv = a.w;
-    wv.off = s_off;
-    if (!kF32 || !a.stage) __syncthreads();
-    if (kF32 && a.stage) {
-        float *sm = reinterpret_cast<float *>(smem);
-        for (int i = threadIdx.x; i < a.stage_box; i += blockDim.x) sm[i] = a.w.box[i];
-        for (int i = threadIdx.x; i < a.stage_prim; i += blockDim.x) {
-            sm[a.stage_box + i] = a.w.prim[i];
-        }
-        __syncthreads();
-        wv.box = sm;
-        if (a.stage_prim) {
-            // staged primitives: the list scans read them here, not the copy
-            wv.prim = sm + a.stage_box;
-            wv.aos = nullptr;
+// Shared memory of one warp: walks that wait, kHeatPool slots, one array per
+// field (doubles first), then the lanes' statistics of the task at hand.
+// Slots from 0 up hold walks whose last step came within the FP32 shell or
+// reached the step cap, with the nearest primitive's wide slot; slots from the
+// last one down walks to be resumed, with their radius.  The derivative sums
+// (five per walk, ten per warp) are there in the adjoint pass only.
+constexpr int kHeatPool = 64;
+
+struct HeatPool {
+    double *d;
+    bool adj;
+    __host__ __device__ static constexpr int doubles(bool adj) {
+        return (adj ? 6 : 1) * kHeatPool + 3 * kHeatPool + 3 * 32 + 32 + (adj ? 10 : 0);
+    }
+    __device__ __forceinline__ double &sample(int i) { return d[i]; }
+    __device__ __forceinline__ double &deriv(int k, int i) { return d[(1 + k) * kHeatPool + i]; }
+    __device__ __forceinline__ unsigned *words() const {
+        return reinterpret_cast<unsigned *>(d + (adj ? 6 : 1) * kHeatPool);
+    }
+    __device__ __forceinline__ int &steps(int i) { return reinterpret_cast<int *>(words())[i]; }
+    __device__ __forceinline__ int &walk(int i) {
+        return reinterpret_cast<int *>(words())[kHeatPool + i];
+    }
+    __device__ __forceinline__ int &slot(int i) {
+        return reinterpret_cast<int *>(words())[2 * kHeatPool + i];
+    }
+    __device__ __forceinline__ float &radius(int i) {
+        return reinterpret_cast<float *>(words())[2 * kHeatPool + i];
+    }
+    __device__ __forceinline__ float &x(int k, int i) {
+        return reinterpret_cast<float *>(words())[(3 + k) * kHeatPool + i];
+    }
+    // per lane: ShiftedSums (k, s, q), then two counts (walks, steps)
+    __device__ __forceinline__ double &sum(int k, int lane) {
+        return d[(adj ? 9 : 4) * kHeatPool + k * 32 + lane];
+    }
+    __device__ __forceinline__ int &count(int k, int lane) {
+        return reinterpret_cast<int *>(&sum(3, 0))[k * 32 + lane];
+    }
+    // adjoint pass, per warp: sums and sums of squares of the derivatives
+    __device__ __forceinline__ double &deriv_sum(int k) { return sum(4, k); }
+};
+
+// Warp merge of a task's lane statistics into its partial.
+__device__ __forceinline__ void write_heat_partial(const HeatArgs &a, unsigned long long task,
+                                                   const ShiftedSums &acc, int steps_acc,
+                                                   unsigned hits, double queries, bool all_steps,
+                                                   bool bad, bool adj, double jsum[5],
+                                                   double jsq[5]) {
+    const int lane = threadIdx.x & 31;
+    if (__ballot_sync(kFull, bad) && lane == 0) atomicOr(&a.ctr->error_flags, kErrBadState);
+    double n_tot = static_cast<double>(acc.n);
+    double mean_acc, m2_acc;
+    acc.finish(mean_acc, m2_acc);
+    unsigned long long steps_tot = static_cast<unsigned long long>(steps_acc);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        const double nb = __shfl_down_sync(kFull, n_tot, o);
+        const double mb = __shfl_down_sync(kFull, mean_acc, o);
+        const double m2b = __shfl_down_sync(kFull, m2_acc, o);
+        const unsigned long long sb = __shfl_down_sync(kFull, steps_tot, o);
+        const unsigned hb = __shfl_down_sync(kFull, hits, o);
+        chan_merge(n_tot, mean_acc, m2_acc, nb, mb, m2b);
+        steps_tot += sb;
+        hits += hb;
+    }
+    if (adj) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+#pragma unroll
+            for (int k = 0; k < 5; ++k) {
+                jsum[k] += __shfl_down_sync(kFull, jsum[k], o);
+                jsq[k] += __shfl_down_sync(kFull, jsq[k], o);
+            }
         }
     }
+    if (lane == 0) {
+        HeatPartial hp;
+        hp.n = n_tot;
+        hp.mean = mean_acc;
+        hp.m2 = m2_acc;
+        hp.steps = static_cast<double>(steps_tot);
+        hp.queries = all_steps ? static_cast<double>(steps_tot) : queries;
+        hp.hits = hits;
+        hp.pad = 0;
+#pragma unroll
+        for (int k = 0; k < 5; ++k) {
+            hp.jsum[k] = jsum[k];
+            hp.jsq[k] = jsq[k];
+        }
+        a.partials[task] = hp;
+    }
+}
+
+// One FAST_FP32 task.  Half of these walks' steps query (epsilon is small),
+// so the lists and cooperative queries run in every iteration, for about half
+// of the lanes; but the FP64 re-projection of a step that came within the FP32
+// shell and what ends a walk concern one or two.  Such walks wait in the
+// warp's pool while their lanes step others, and 32 of them are re-projected
+// together; those that go on return to the lanes (fast_task32 in
+// kernels_fast.cu explains the pool and why it cannot overflow).  Slab of 20k
+// triangles, 4096 probes x 2048 walks, forward / adjoint pass: 20.1 / 20.4 ->
+// 17.4 / 19.5 ms; disk of 2000 segments 1.85 / 1.94 -> 1.32 / 1.56 ms.
+template <int DIM, int HC>
+__device__ __forceinline__ void heat_task32(const HeatArgs &a, const WideView &wv,
+                                            unsigned long long task, long long pidx, int c,
+                                            double *s_pool) {
     const int lane = threadIdx.x & 31;
     const unsigned lt_mask = (1u << lane) - 1u;
     const double eps = a.eps;
     const bool adj = a.adjoint != 0;
+    HeatPool pool{s_pool, adj};
+
+    double px0, py0, pz0;
+    uint64_t linear;
+    point_at(a.ps, pidx, px0, py0, pz0, linear);
+    const uint64_t pseed = point_seed(a.seed, linear);
+    const V3<float> p0{static_cast<float>(px0), static_cast<float>(py0), static_cast<float>(pz0)};
+    const StartRecord st0 = a.start[pidx];
+    const float R0 = static_cast<float>(st0.radius);
+    const double cgrad = adj ? a.grad_u[pidx] / static_cast<double>(a.n_walks) : 0.0;
+    const int w0 = c * a.chunk;
+    const int w1 = min(a.n_walks, w0 + a.chunk);
+
+    for (int k = 0; k < 2; ++k) pool.count(k, lane) = 0;
+    if (adj && lane < 10) pool.deriv_sum(lane) = 0.0;
+    auto finish = [&](double value, int steps) {
+        const int n = pool.count(0, lane);
+        ShiftedSums acc;
+        acc.n = n;
+        if (n > 0) {
+            acc.k = pool.sum(0, lane);
+            acc.s = pool.sum(1, lane);
+            acc.q = pool.sum(2, lane);
+        } else {
+            pool.sum(0, lane) = value;
+        }
+        acc.add(value);
+        pool.sum(1, lane) = acc.s;
+        pool.sum(2, lane) = acc.q;
+        pool.count(0, lane) = acc.n;
+        pool.count(1, lane) += steps;
+    };
+    unsigned hits = 0;
+    unsigned queries = 0;  // BVH queries of this task (warp-uniform; < 2^32)
+    bool bad = false;      // a closest-point query found no primitive
+
+    const bool start_stops = !(st0.radius > eps);
+    if (start_stops) {
+        // the start point is inside the shell: every walk ends there
+        for (int w = w0 + lane; w < w1; w += 32) {
+            finish(st0.slot >= 0 ? boundary_data<DIM>(a, st0.slot,
+                                                      V3<double>{st0.nx, st0.ny, st0.nz}, cgrad)
+                                 : 0.0,
+                   0);
+        }
+    }
+
+    bool active = false;
+    int walk = 0, steps = 0;
+    V3<float> p = p0;
+    float R = R0;
+    double sample = 0.0;
+    double j[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
+    int next = start_stops ? w1 : w0;
+    int waiting = 0, resume = 0;
+    const uint2 pkey = PhiloxStream::key_of(pseed);
+
+    for (;;) {
+        // lanes without a walk take one: a resumed walk, else a new one
+        const unsigned empty = __ballot_sync(kFull, !active);
+        if (empty) {
+            if (!active) {
+                const int rank = __popc(empty & lt_mask);
+                if (rank < resume) {
+                    const int i = kHeatPool - resume + rank;
+                    steps = pool.steps(i);
+                    walk = pool.walk(i);
+                    R = pool.radius(i);
+                    p = V3<float>{pool.x(0, i), pool.x(1, i), DIM == 3 ? pool.x(2, i) : 0.0f};
+                    sample = pool.sample(i);
+                    if (adj) {
+#pragma unroll
+                        for (int k = 0; k < 5; ++k) j[k] = pool.deriv(k, i);
+                    }
+                    active = true;
+                } else {
+                    walk = next + rank - resume;
+                    active = walk < w1;
+                    p = p0;
+                    R = R0;
+                    sample = 0.0;
+#pragma unroll
+                    for (int k = 0; k < 5; ++k) j[k] = 0.0;
+                    steps = 0;
+                }
+            }
+            const int taken = __popc(empty);
+            next = min(next + max(taken - resume, 0), w1);
+            resume = max(resume - taken, 0);
+            __syncwarp();
+        }
+        // one step of every walk in flight
+        bool need_query = false;
+        bool listed = false;  // answered from a near-boundary list
+        int packed = -1;      // the list
+        int slot = -1;        // winner of the step's query
+        if (active) {
+            FastRng<float> rng(pkey, static_cast<uint32_t>(walk));
+            rng.begin_step(steps);
+            sample += heat_source<DIM, float>(a, p, R, rng, adj, j);
+            p = sphere_step<DIM, false, float>(p, R, rng);
+            ++steps;
+            need_query = true;
+            // the walk kernels' lattice step: away from the shell a
+            // lattice lower bound is the radius (forward and replay
+            // take the same branches, the lattice is fixed)
+            if (wv.gd != nullptr && steps < a.max_steps) {
+                const LatticeSample ls = lattice_sample<DIM>(wv, p.x, p.y, DIM == 3 ? p.z : 0.0f);
+                const float gb = (ls.d - ls.r) * a.shrink;
+                if (ls.d >= wv.gratio * ls.r && gb > 0.0f && gb * gb > a.shell2) {
+                    R = gb;
+                    need_query = false;
+                } else if (ls.d <= a.list_t) {
+                    // near the boundary: a query over the node's candidate
+                    // list, when it has one (2D: this lane scans it; 3D:
+                    // the warp, below)
+                    const int2 e = __ldg(wv.gl + ls.node);
+                    packed = DIM == 3 && e.x >= 0 ? list_prefix(wv, e, ls.r) : e.x;
+                    listed = packed >= 0;
+                    need_query = !listed;
+                }
+            }
+        }
+        float qbest = 0.0f;
+        if constexpr (DIM == 2) {
+            if (listed) {
+                const WideResult q = list_nearest<DIM>(wv, list_of(wv, packed),
+                                                       list_length(packed), p.x, p.y, 0.0f);
+                qbest = q.best;
+                slot = q.slot;
+            }
+        } else if (__any_sync(kFull, listed)) {
+            const WideResult q = warp_list_nearest<DIM>(wv, listed, packed, p.x, p.y, p.z);
+            if (listed) {
+                qbest = q.best;
+                slot = q.slot;
+            }
+        }
+        unsigned pending = __ballot_sync(kFull, need_query);
+        queries += __popc(pending) + __popc(__ballot_sync(kFull, listed));
+        while (pending) {
+            const int jl = __ffs(pending) - 1;
+            pending &= pending - 1u;
+            const float qx = __shfl_sync(kFull, p.x, jl);
+            const float qy = __shfl_sync(kFull, p.y, jl);
+            const float qz = DIM == 3 ? __shfl_sync(kFull, p.z, jl) : 0.0f;
+            const WideResult r = wide_nearest<DIM, HC>(wv, qx, qy, qz, a.keep, a.exact2);
+            if (lane == jl) {
+                qbest = r.best;
+                slot = r.slot;
+            }
+        }
+        bool defer = false;
+        if (need_query || listed) {
+            const float r = sqrtf(qbest);
+            R = qbest > a.shell2 ? r * a.shrink : r;
+            defer = R * R <= a.shell2 || steps >= a.max_steps;
+        }
+        const unsigned put = __ballot_sync(kFull, defer);
+        if (put) {
+            if (defer) {
+                const int i = waiting + __popc(put & lt_mask);
+                pool.steps(i) = steps;
+                pool.walk(i) = walk;
+                // a walk at the step cap outside the shell: no re-projection
+                // may resume it (its slot is marked)
+                pool.slot(i) = R * R <= a.shell2 ? slot : ~slot - 1;
+                pool.x(0, i) = p.x;
+                pool.x(1, i) = p.y;
+                if (DIM == 3) pool.x(2, i) = p.z;
+                pool.sample(i) = sample;
+                if (adj) {
+#pragma unroll
+                    for (int k = 0; k < 5; ++k) pool.deriv(k, i) = j[k];
+                }
+                active = false;
+            }
+            waiting += __popc(put);
+            __syncwarp();
+        }
+        const bool idle = !__any_sync(kFull, active);
+        if (idle && waiting == 0 && resume == 0 && next >= w1) break;
+        if (waiting < 32 && !(idle && next >= w1 && resume == 0)) continue;
+
+        // ---- re-projection and endings, one waiting walk per lane
+        const int m = min(waiting, 32);
+        waiting -= m;
+        const int i = waiting + lane;
+        bool go_on = false, ended = false;
+        float qR = 0.0f;
+        V3<float> q{0.0f, 0.0f, 0.0f};
+        int qsteps = 0, qwalk = 0;
+        double qsample = 0.0;
+        double qj[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
+        if (lane < m) {
+            qsteps = pool.steps(i);
+            qwalk = pool.walk(i);
+            int s = pool.slot(i);
+            const bool capped = s < -1;
+            if (capped) s = ~(s + 1);
+            q = V3<float>{pool.x(0, i), pool.x(1, i), DIM == 3 ? pool.x(2, i) : 0.0f};
+            qsample = pool.sample(i);
+            if (adj) {
+#pragma unroll
+                for (int k = 0; k < 5; ++k) qj[k] = pool.deriv(k, i);
+            }
+            bool stop = false;
+            V3<double> np{0.0, 0.0, 0.0};
+            int bid = -1;
+            int bslot = -1;
+            if (s < 0) {  // a query found no primitive: flag it, stop
+                bad = true;
+                if (capped) ++hits;
+                stop = true;
+            } else {
+                bslot = wv.wide2bin[s];
+                const double d2 = reproject64_sq<DIM>(
+                    a.s, bslot, static_cast<double>(q.x), static_cast<double>(q.y),
+                    static_cast<double>(q.z), np, bid);
+                if (!capped && d2 <= eps * eps) {
+                    stop = true;
+                } else {
+                    qR = static_cast<float>(sqrt(d2));
+                    if (qsteps >= a.max_steps) {
+                        ++hits;
+                        stop = true;
+                    }
+                }
+            }
+            if (stop) {
+                finish(qsample + (bslot >= 0 ? boundary_data<DIM>(a, bslot, np, cgrad) : 0.0),
+                       qsteps);
+            }
+            go_on = !stop;
+            ended = stop;
+        }
+        if (adj) {
+            // the ended walks' derivatives, summed over the warp
+#pragma unroll
+            for (int k = 0; k < 5; ++k) {
+                double v = ended ? qj[k] : 0.0, v2 = v * v;
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) {
+                    v += __shfl_xor_sync(kFull, v, o);
+                    v2 += __shfl_xor_sync(kFull, v2, o);
+                }
+                if (lane == 0) {
+                    pool.deriv_sum(k) += v;
+                    pool.deriv_sum(5 + k) += v2;
+                }
+            }
+        }
+        const unsigned back = __ballot_sync(kFull, go_on);
+        if (back) {
+            if (go_on) {
+                const int k2 = kHeatPool - 1 - resume - __popc(back & lt_mask);
+                pool.steps(k2) = qsteps;
+                pool.walk(k2) = qwalk;
+                pool.radius(k2) = qR;
+                pool.x(0, k2) = q.x;
+                pool.x(1, k2) = q.y;
+                if (DIM == 3) pool.x(2, k2) = q.z;
+                pool.sample(k2) = qsample;
+                if (adj) {
+#pragma unroll
+                    for (int k = 0; k < 5; ++k) pool.deriv(k, k2) = qj[k];
+                }
+            }
+            resume += __popc(back);
+            __syncwarp();
+        }
+    }
+
+    ShiftedSums acc;
+    acc.n = pool.count(0, lane);
+    if (acc.n > 0) {
+        acc.k = pool.sum(0, lane);
+        acc.s = pool.sum(1, lane);
+        acc.q = pool.sum(2, lane);
+    }
+    double jsum[5] = {0.0, 0.0, 0.0, 0.0, 0.0}, jsq[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
+    if (adj && lane == 0) {
+#pragma unroll
+        for (int k = 0; k < 5; ++k) {
+            jsum[k] = pool.deriv_sum(k);
+            jsq[k] = pool.deriv_sum(5 + k);
+        }
+    }
+    write_heat_partial(a, task, acc, pool.count(1, lane), hits, static_cast<double>(queries),
+                       false, bad, adj, jsum, jsq);
+    __syncwarp();
+}
+
+// One FAST_FP64 task: every step queries in FP64, by the whole warp where
+// the scene allows it (wide64.cuh; slab of 20k triangles, 256 probes x 256
+// walks: 16.8 -> 3.3 ms).
+template <int DIM>
+__device__ __forceinline__ void heat_task64(const HeatArgs &a, const WideView &wv,
+                                            unsigned long long task, long long pidx, int c) {
+    const int lane = threadIdx.x & 31;
+    const unsigned lt_mask = (1u << lane) - 1u;
+    const double eps = a.eps;
+    const bool adj = a.adjoint != 0;
+
+    V3<double> p0;
+    uint64_t linear;
+    point_at(a.ps, pidx, p0.x, p0.y, p0.z, linear);
+    const uint64_t pseed = point_seed(a.seed, linear);
+    const StartRecord st0 = a.start[pidx];
+    const double R0 = st0.radius;
+    const bool start_stops = !(R0 > eps);
+    const double cgrad = adj ? a.grad_u[pidx] / static_cast<double>(a.n_walks) : 0.0;
+    const int w0 = c * a.chunk;
+    const int w1 = min(a.n_walks, w0 + a.chunk);
+
+    int steps_acc = 0;
+    ShiftedSums acc;
+    double jsum[5] = {0.0, 0.0, 0.0, 0.0, 0.0}, jsq[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
+    unsigned hits = 0;
+
+    int walk = w0 + lane;
+    bool active = walk < w1;
+    int next = w0 + 32;
+    V3<double> p = p0;
+    double R = R0;
+    double sample = 0.0;
+    double j[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
+    int steps = 0;
+    int slot = -1;  // binary slot of the last query
+    V3<double> np{0.0, 0.0, 0.0};
+    const uint2 pkey = PhiloxStream::key_of(pseed);
+    FastRng<double> rng(pkey, static_cast<uint32_t>(walk));
+
+    while (__any_sync(kFull, active)) {
+        // one step of every walk in flight (none from a start point inside
+        // the shell)
+        const bool query = active && !start_stops;
+        if (query) {
+            rng.begin_step(steps);
+            sample += heat_source<DIM, double>(a, p, R, rng, adj, j);
+            p = sphere_step<DIM, false, double>(p, R, rng);
+            ++steps;
+        }
+        if (wv.margin64 >= 0.0f && wv.n > thread_query_prims(DIM)) {
+            Candidates cand{0, -1};
+            unsigned pending = __ballot_sync(kFull, query);
+            while (pending) {
+                const int jl = __ffs(pending) - 1;
+                pending &= pending - 1u;
+                const double qx = __shfl_sync(kFull, p.x, jl);
+                const double qy = __shfl_sync(kFull, p.y, jl);
+                const double qz = DIM == 3 ? __shfl_sync(kFull, p.z, jl) : 0.0;
+                const Candidates found = warp_candidates64<DIM>(a.s, wv, qx, qy, qz);
+                if (lane == jl) cand = found;
+            }
+            if (query) {
+                R = sqrt(pick_nearest64<DIM>(a.s, cand, p.x, p.y, p.z, slot, np.x, np.y, np.z));
+            }
+        } else if (query) {
+            const Nearest<double> q = nearest64<DIM>(a.s, p.x, p.y, p.z, dinf());
+            R = sqrt(q.best);
+            np = V3<double>{q.x, q.y, q.z};
+            slot = q.slot;
+        }
+        // walks whose new radius is in the shell, or that reached the step
+        // cap, end in the iteration of their last step
+        bool done = active && (start_stops || !(R > eps));
+        if (active && !done && steps >= a.max_steps) {
+            ++hits;
+            done = true;
+        }
+        if (done) {
+            if (start_stops) {
+                np = V3<double>{st0.nx, st0.ny, st0.nz};
+                slot = st0.slot;
+            }
+            acc.add(sample + (slot >= 0 ? boundary_data<DIM>(a, slot, np, cgrad) : 0.0));
+            steps_acc += steps;
+            if (adj) {
+#pragma unroll
+                for (int k = 0; k < 5; ++k) {
+                    jsum[k] += j[k];
+                    jsq[k] += j[k] * j[k];
+                }
+            }
+        }
+        const unsigned done_mask = __ballot_sync(kFull, done);
+        if (done_mask) {
+            if (done) {
+                walk = next + __popc(done_mask & lt_mask);
+                active = walk < w1;
+                if (active) {
+                    p = p0;
+                    R = R0;
+                    sample = 0.0;
+#pragma unroll
+                    for (int k = 0; k < 5; ++k) j[k] = 0.0;
+                    steps = 0;
+                    rng = FastRng<double>(pkey, static_cast<uint32_t>(walk));
+                }
+            }
+            next += __popc(done_mask);
+        }
+    }
+    write_heat_partial(a, task, acc, steps_acc, hits, 0.0, true, false, adj, jsum, jsq);
+}
+
+template <int DIM, typename T, int MIN_BLOCKS, int HC>
+__global__ void __launch_bounds__(256, MIN_BLOCKS) heat_walk_kernel(HeatArgs a) {
+    constexpr bool kF32 = std::is_same<T, float>::value;
+    extern __shared__ float4 smem[];  // FP32: the warps' pools, then the staged scene
+    __shared__ int s_off[8];
+    if (threadIdx.x < 8) s_off[threadIdx.x] = a.w.off[threadIdx.x];
+    WideView wv = a.w;
+    wv.off = s_off;
+    double *pool = nullptr;
+    if constexpr (kF32) {
+        const int words = HeatPool::doubles(a.adjoint != 0);
+        pool = reinterpret_cast<double *>(smem) + (threadIdx.x >> 5) * words;
+        if (a.stage) {
+            float *sm = reinterpret_cast<float *>(reinterpret_cast<double *>(smem) + 8 * words);
+            for (int i = threadIdx.x; i < a.stage_box; i += blockDim.x) sm[i] = a.w.box[i];
+            for (int i = threadIdx.x; i < a.stage_prim; i += blockDim.x) {
+                sm[a.stage_box + i] = a.w.prim[i];
+            }
+            wv.box = sm;
+            if (a.stage_prim) {
+                // staged primitives: the list scans read them here, not the copy
+                wv.prim = sm + a.stage_box;
+                wv.aos = nullptr;
+            }
+        }
+    }
+    __syncthreads();
+    const int lane = threadIdx.x & 31;
 
     for (;;) {
         unsigned long long task = 0;
@@ -246,268 +764,10 @@ __global__ void __launch_bounds__(256, MIN_BLOCKS) heat_walk_kernel(HeatArgs a) 
         const long long pidx = static_cast<long long>(task / a.chunks);
         const int c = static_cast<int>(task % a.chunks);
         if (a.location[pidx] != 1) continue;
-
-        double px0, py0, pz0;
-        uint64_t linear;
-        point_at(a.ps, pidx, px0, py0, pz0, linear);
-        const uint64_t pseed = point_seed(a.seed, linear);
-        const V3<T> p0{static_cast<T>(px0), static_cast<T>(py0), static_cast<T>(pz0)};
-        const StartRecord st0 = a.start[pidx];
-        const T R0 = static_cast<T>(st0.radius);
-        const bool start_stops = !(st0.radius > eps);
-        const double cgrad = adj ? a.grad_u[pidx] / static_cast<double>(a.n_walks) : 0.0;
-        const int w0 = c * a.chunk;
-        const int w1 = min(a.n_walks, w0 + a.chunk);
-
-        int steps_acc = 0;
-        ShiftedSums acc;
-        // per-lane sums and sums of squares of the derivatives, in shared
-        // memory (touched once per finished walk) to keep registers for the walk
-        if (adj) {
-#pragma unroll
-            for (int k = 0; k < 10; ++k) s_acc[k][threadIdx.x] = 0.0;
-        }
-        unsigned hits = 0;
-        unsigned queries = 0;  // BVH queries of this task (FP32; warp-uniform; < 2^32)
-        bool bad = false;  // a closest-point query found no primitive
-
-        int walk = w0 + lane;
-        bool active = walk < w1;
-        int next = w0 + 32;
-        V3<T> p = p0;
-        T R = R0;
-        double sample = 0.0;
-        double j[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
-        int steps = 0;
-        int slot = -1;                    // FP32: wide slot of the last query
-        int slot64 = -1;                  // FP64: binary slot of the last query
-        V3<double> np64{0.0, 0.0, 0.0};
-        const uint2 pkey = PhiloxStream::key_of(pseed);
-        FastRng<T> rng(pkey, static_cast<uint32_t>(walk));
-
-        while (__any_sync(kFull, active)) {
-            bool need_query = false;
-            bool listed = false;  // answered from a near-boundary list
-            int packed = -1;      // 3D: the list the warp scans for this lane
-            // one step of every walk in flight (none from a start point
-            // inside the shell)
-            if (active && !start_stops) {
-                rng.begin_step(steps);
-                sample += heat_source<DIM, T>(a, p, R, rng, adj, j);
-                p = sphere_step<DIM, false, T>(p, R, rng);
-                ++steps;
-                if constexpr (kF32) {
-                    need_query = true;
-                    // the walk kernels' lattice step: away from the shell a
-                    // lattice lower bound is the radius (forward and replay
-                    // take the same branches, the lattice is fixed)
-                    if (wv.gd != nullptr && steps < a.max_steps) {
-                        const LatticeSample ls =
-                            lattice_sample<DIM>(wv, p.x, p.y, DIM == 3 ? p.z : 0.0f);
-                        const float gb = (ls.d - ls.r) * a.shrink;
-                        if (ls.d >= wv.gratio * ls.r && gb > 0.0f && gb * gb > a.shell2) {
-                            R = gb;
-                            need_query = false;
-                        } else if (ls.d <= a.list_t) {
-                            // near the boundary: a query over the node's
-                            // candidate list, when it has one (2D: this
-                            // lane scans it; 3D: the warp, below)
-                            const int2 e = __ldg(wv.gl + ls.node);
-                            const int v = DIM == 3 && e.x >= 0 ? list_prefix(wv, e, ls.r) : e.x;
-                            if (v >= 0) {
-                                if constexpr (DIM == 2) {
-                                    const WideResult q = list_nearest<DIM>(
-                                        wv, list_of(wv, v), list_length(v),
-                                        static_cast<float>(p.x), static_cast<float>(p.y), 0.0f);
-                                    const float r = sqrtf(q.best);
-                                    R = static_cast<T>(q.best > a.shell2 ? r * a.shrink : r);
-                                    slot = q.slot;
-                                } else {
-                                    packed = v;
-                                }
-                                need_query = false;
-                                listed = true;
-                            }
-                        }
-                    }
-                } else {
-                    const Nearest<double> q = nearest64<DIM>(
-                        a.s, static_cast<double>(p.x), static_cast<double>(p.y),
-                        static_cast<double>(p.z), dinf());
-                    R = static_cast<T>(sqrt(q.best));
-                    np64 = V3<double>{q.x, q.y, q.z};
-                    slot64 = q.slot;
-                }
-            }
-            if constexpr (kF32 && DIM == 3) {
-                const bool want = packed >= 0;
-                if (__any_sync(kFull, want)) {
-                    const WideResult q = warp_list_nearest<DIM>(
-                        wv, want, packed, static_cast<float>(p.x), static_cast<float>(p.y),
-                        static_cast<float>(p.z));
-                    if (want) {
-                        const float r = sqrtf(q.best);
-                        R = static_cast<T>(q.best > a.shell2 ? r * a.shrink : r);
-                        slot = q.slot;
-                    }
-                }
-            }
-            if constexpr (kF32) {
-                unsigned pending = __ballot_sync(kFull, need_query);
-                queries += __popc(pending) + __popc(__ballot_sync(kFull, listed));
-                float qbest = 0.0f;
-                int qslot = -1;
-                while (pending) {
-                    const int jl = __ffs(pending) - 1;
-                    pending &= pending - 1u;
-                    const float qx = __shfl_sync(kFull, static_cast<float>(p.x), jl);
-                    const float qy = __shfl_sync(kFull, static_cast<float>(p.y), jl);
-                    const float qz =
-                        DIM == 3 ? __shfl_sync(kFull, static_cast<float>(p.z), jl) : 0.0f;
-                    const WideResult r = wide_nearest<DIM, HC>(wv, qx, qy, qz, a.keep, a.exact2);
-                    if (lane == jl) {
-                        qbest = r.best;
-                        qslot = r.slot;
-                    }
-                }
-                if (need_query) {
-                    const float r = sqrtf(qbest);
-                    R = static_cast<T>(qbest > a.shell2 ? r * a.shrink : r);
-                    slot = qslot;
-                }
-            }
-            // walks whose new radius is in the shell, or that reached the
-            // step cap, end in the iteration of their last step
-            bool done = false;
-            double value = 0.0;
-            if (active) {
-                bool stop = false;
-                V3<double> np{0.0, 0.0, 0.0};
-                int bslot = -1;
-                int bid = -1;
-                if (start_stops) {
-                    stop = true;
-                    np = V3<double>{st0.nx, st0.ny, st0.nz};
-                    bslot = st0.slot;
-                } else if (!kF32) {
-                    stop = !(static_cast<double>(R) > eps);
-                    np = np64;
-                    bslot = slot64;
-                } else if (static_cast<float>(R) * static_cast<float>(R) <= a.shell2) {
-                    if (slot < 0) {  // a query found no primitive: flag it, stop
-                        bad = true;
-                        stop = true;
-                    } else {
-                        bslot = wv.wide2bin[slot];
-                        const double d2 = reproject64_sq<DIM>(
-                            a.s, bslot, static_cast<double>(p.x), static_cast<double>(p.y),
-                            static_cast<double>(p.z), np, bid);
-                        if (d2 <= eps * eps) {
-                            stop = true;
-                        } else {
-                            R = static_cast<T>(sqrt(d2));
-                        }
-                    }
-                }
-                if (!stop && steps >= a.max_steps) {
-                    ++hits;
-                    stop = true;
-                    if (kF32) {
-                        if (slot < 0) {
-                            bad = true;
-                        } else {
-                            bslot = wv.wide2bin[slot];
-                            reproject64<DIM>(a.s, bslot, static_cast<double>(p.x),
-                                             static_cast<double>(p.y), static_cast<double>(p.z),
-                                             np, bid);
-                        }
-                    } else {
-                        np = np64;
-                        bslot = slot64;
-                    }
-                }
-                if (stop) {
-                    value = sample + (bslot >= 0 ? boundary_data<DIM>(a, bslot, np, cgrad) : 0.0);
-                    done = true;
-                }
-            }
-            if (done) {
-                acc.add(value);
-                steps_acc += steps;
-                if (adj) {
-#pragma unroll
-                    for (int k = 0; k < 5; ++k) {
-                        s_acc[k][threadIdx.x] += j[k];
-                        s_acc[5 + k][threadIdx.x] += j[k] * j[k];
-                    }
-                }
-            }
-            const unsigned done_mask = __ballot_sync(kFull, done);
-            if (done_mask) {
-                if (done) {
-                    walk = next + __popc(done_mask & lt_mask);
-                    active = walk < w1;
-                    if (active) {
-                        p = p0;
-                        R = R0;
-                        sample = 0.0;
-#pragma unroll
-                        for (int k = 0; k < 5; ++k) j[k] = 0.0;
-                        steps = 0;
-                        rng = FastRng<T>(pkey, static_cast<uint32_t>(walk));
-                    }
-                }
-                next += __popc(done_mask);
-            }
-        }
-
-        if (__ballot_sync(kFull, bad) && lane == 0) atomicOr(&a.ctr->error_flags, kErrBadState);
-        double n_tot = static_cast<double>(acc.n);
-        double mean_acc, m2_acc;
-        acc.finish(mean_acc, m2_acc);
-        unsigned long long steps_tot = static_cast<unsigned long long>(steps_acc);
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            const double nb = __shfl_down_sync(kFull, n_tot, o);
-            const double mb = __shfl_down_sync(kFull, mean_acc, o);
-            const double m2b = __shfl_down_sync(kFull, m2_acc, o);
-            const unsigned long long sb = __shfl_down_sync(kFull, steps_tot, o);
-            const unsigned hb = __shfl_down_sync(kFull, hits, o);
-            chan_merge(n_tot, mean_acc, m2_acc, nb, mb, m2b);
-            steps_tot += sb;
-            hits += hb;
-        }
-        double jsum[5] = {0.0, 0.0, 0.0, 0.0, 0.0}, jsq[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
-        if (adj) {
-#pragma unroll
-            for (int k = 0; k < 5; ++k) {
-                jsum[k] = s_acc[k][threadIdx.x];
-                jsq[k] = s_acc[5 + k][threadIdx.x];
-            }
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) {
-#pragma unroll
-                for (int k = 0; k < 5; ++k) {
-                    jsum[k] += __shfl_down_sync(kFull, jsum[k], o);
-                    jsq[k] += __shfl_down_sync(kFull, jsq[k], o);
-                }
-            }
-        }
-        if (lane == 0) {
-            HeatPartial hp;
-            hp.n = n_tot;
-            hp.mean = mean_acc;
-            hp.m2 = m2_acc;
-            hp.steps = static_cast<double>(steps_tot);
-            hp.queries = kF32 ? static_cast<double>(queries) : static_cast<double>(steps_tot);
-            hp.hits = hits;
-            hp.pad = 0;
-#pragma unroll
-            for (int k = 0; k < 5; ++k) {
-                hp.jsum[k] = jsum[k];
-                hp.jsq[k] = jsq[k];
-            }
-            a.partials[task] = hp;
+        if constexpr (kF32) {
+            heat_task32<DIM, HC>(a, wv, task, pidx, c, pool);
+        } else {
+            heat_task64<DIM>(a, wv, task, pidx, c);
         }
     }
 }
@@ -612,24 +872,23 @@ cudaError_t launch_heat_dim(const HeatArgs &a, int precision, const FastPlan &pl
         // forward and replay read the same tree, so they use one instantiation
         return with_height_class(height_class(a.w.H), [&](auto h) -> cudaError_t {
             constexpr int HC = decltype(h)::value;
-            // 4 blocks / SM (64 registers) for the height <= 3 traversals:
-            // the kernel waits on loads, so more resident warps pay
-            constexpr int kMinBlocks = (HC == kHeightUpTo2 || HC == kHeight3) ? 4 : 3;
-            auto k = heat_walk_kernel<DIM, float, kMinBlocks, HC>;
-            // the static accumulators (20 KB) plus the staged scene can pass
-            // the 48 KB default: opt in whenever anything is staged
-            if (plan.smem_bytes > 0) {
-                cudaError_t e = cudaFuncSetAttribute(
-                    k, cudaFuncAttributeMaxDynamicSharedMemorySize, plan.smem_bytes);
-                if (e != cudaSuccess) return e;
-            }
-            cudaError_t e = grid_for(k, plan.smem_bytes, blocks);
+            // 4 blocks / SM (64 registers): the kernel waits on loads, so
+            // resident warps pay in spite of spills (slab of 20k triangles,
+            // forward / adjoint pass: 17.4 / 19.5 ms, 19.0 / 20.1 at 3)
+            auto k = heat_walk_kernel<DIM, float, 4, HC>;
+            // the warps' pools (24 KB, adjoint pass 46 KB) and the staged scene
+            const int smem =
+                plan.smem_bytes + 8 * 8 * HeatPool::doubles(a.adjoint != 0);
+            cudaError_t e = cudaFuncSetAttribute(
+                k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
             if (e != cudaSuccess) return e;
-            k<<<blocks, plan.threads, plan.smem_bytes, stream>>>(a);
+            e = grid_for(k, smem, blocks);
+            if (e != cudaSuccess) return e;
+            k<<<blocks, plan.threads, smem, stream>>>(a);
             return cudaGetLastError();
         });
     } else {
-        auto k = heat_walk_kernel<DIM, double, 1, kHeightAny>;
+        auto k = heat_walk_kernel<DIM, double, 2, kHeightAny>;
         cudaError_t e = grid_for(k, 0, blocks);
         if (e != cudaSuccess) return e;
         k<<<blocks, plan.threads, 0, stream>>>(a);
