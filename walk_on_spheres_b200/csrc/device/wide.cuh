@@ -384,12 +384,19 @@ __device__ int wide_range(const WideView &w, float px, float py, float pz, float
 // hot ones).  kHeightAny keeps every path.  kLaneScan: at most kLanePrims
 // primitives, which the walk kernels scan lane by lane (lane_nearest);
 // wide_nearest treats it like kHeightUpTo2.
-enum : int { kHeightAny = -1, kHeightOther = 0, kLaneScan = 1, kHeightUpTo2 = 2, kHeight3 = 3 };
+enum : int {
+    kHeightAny = -1,
+    kHeightOther = 0,
+    kLaneScan = 1,
+    kHeightUpTo2 = 2,
+    kHeight3 = 3,
+    kHeight4 = 4
+};
 
 __host__ __device__ __forceinline__ int lane_prims(int dim) { return dim == 2 ? 64 : 32; }
 
 __host__ __device__ __forceinline__ int height_class(int H) {
-    return H <= 2 ? kHeightUpTo2 : (H == 3 ? kHeight3 : kHeightOther);
+    return H <= 2 ? kHeightUpTo2 : (H == 3 ? kHeight3 : (H == 4 ? kHeight4 : kHeightOther));
 }
 
 __host__ __device__ __forceinline__ int traversal_class(const WideView &w) {
@@ -403,6 +410,7 @@ inline auto with_height_class(int hc, F &&f) {
         case kLaneScan: return f(std::integral_constant<int, kLaneScan>{});
         case kHeightUpTo2: return f(std::integral_constant<int, kHeightUpTo2>{});
         case kHeight3: return f(std::integral_constant<int, kHeight3>{});
+        case kHeight4: return f(std::integral_constant<int, kHeight4>{});
         default: return f(std::integral_constant<int, kHeightOther>{});
     }
 }
@@ -470,7 +478,7 @@ __device__ __forceinline__ WideResult wide_nearest(const WideView &w, float px, 
         return WideResult{best, slot};
     }
     }
-    if constexpr (HC == kHeightOther || HC == kHeightAny) {
+    if constexpr (HC == kHeight4 || HC == kHeightAny) {
     if (w.H == 4) {
         const float d3 = wide_box_dist<DIM>(w, 3, 0, px, py, pz);
         unsigned m3 = __ballot_sync(kAll, d3 < limit);
@@ -493,6 +501,8 @@ __device__ __forceinline__ WideResult wide_nearest(const WideView &w, float px, 
         }
         return WideResult{best, slot};
     }
+    }
+    if constexpr (HC == kHeightOther || HC == kHeightAny) {
     int h = w.H;    // height of the current node
     int node = 0;   // its index at that height
     float d = wide_box_dist<DIM>(w, h - 1, node, px, py, pz);

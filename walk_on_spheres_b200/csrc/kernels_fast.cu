@@ -564,7 +564,7 @@ constexpr int pool_words() {
 // (star of 777 segments, screened, Green: 3.89 -> 3.78 ms, uniform 2.65 -> 2.35).
 template <class Eq, int HC>
 constexpr int min_blocks32() {
-    return (HC == kHeightUpTo2 || HC == kHeight3) && !HasBalls<Eq>::value ? 4 : 3;
+    return (HC == kHeightUpTo2 || HC == kHeight3 || HC == kHeight4) && !HasBalls<Eq>::value ? 4 : 3;
 }
 
 // Blocks per SM of the FP64 walk kernels (80 / 128 registers at 3 / 2): their
