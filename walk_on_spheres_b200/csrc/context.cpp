@@ -523,7 +523,7 @@ int wos_context::run(const wos_params &p, const PointSet &ps, Fields out,
         fs.exact_below = std::max(eps, btol);
         fs.margin = fp32_distance_margin(scene.bbox, dim);
     }
-    WOS_CUDA(this, launch_classify(view, ps, p.seed, p.max_ray_attempts, btol,
+    WOS_CUDA(this, launch_classify(view, wide, ps, p.seed, p.max_ray_attempts, btol,
                                    eq, out, loc, st, ctr, stream, fs),
              "classification kernel");
     WOS_CUDA(this, cudaEventRecord(events[1], stream), "event");

@@ -416,8 +416,10 @@ enum : int { kMiss = 0, kHit = 1, kAmbiguous = 2 };
 
 // Moller-Trumbore with the reference's ambiguity bands, src/inside.cpp:140-182.
 // a = v0, edge1 = e1, edge2 = e2 of the Eberly record (equal to b-a, c-a).
+// `grazing`: the ray is within 1e-4 of the triangle's plane direction, so
+// rounding may move the crossing by more than the box padding.
 __device__ __forceinline__ int moller_trumbore(const double *p, const double *ray,
-                                               const double2 *r) {
+                                               const double2 *r, bool &grazing) {
     const double ax = r[0].x, ay = r[0].y, az = r[1].x;
     const double e1x = r[1].y, e1y = r[2].x, e1z = r[2].y;
     const double e2x = r[3].x, e2y = r[3].y, e2z = r[4].x;
@@ -432,6 +434,7 @@ __device__ __forceinline__ int moller_trumbore(const double *p, const double *ra
     const double nz = e1x * e2y - e1y * e2x;
     const double nlen = sqrt(nx * nx + ny * ny + nz * nz);
     const double det_tol = kRayEps * nlen;
+    grazing = fabs(det) <= 1e-4 * nlen;
     if (fabs(det) <= det_tol) {
         if (nlen == 0.0) return kMiss;
         double es = 1.0;
@@ -468,7 +471,8 @@ __device__ __forceinline__ int count_ray_hits(const SceneView &s, const double *
         const int b = leaf_first(j, s.n_prims, s.depth);
         const int e = leaf_first(j + 1, s.n_prims, s.depth);
         for (int k = b; k < e; ++k) {
-            const int h = moller_trumbore(p, ray, s.tri64 + 7 * k);
+            bool grazing;
+            const int h = moller_trumbore(p, ray, s.tri64 + 7 * k, grazing);
             if (h == kAmbiguous) return true;
             if (h == kHit) ++hits;
         }

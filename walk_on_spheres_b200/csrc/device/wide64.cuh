@@ -143,29 +143,50 @@ __device__ __forceinline__ double warp_min_double(double v) {
         (static_cast<unsigned long long>(mh) << 32) | ml));
 }
 
-// The winner among the lanes' candidates (`best`, `slot`: the lane's nearest
-// primitive, slot -1 for none).  Equally near primitives: the lowest slot,
-// except that 2D primitives of different boundaries (a corner where two
-// boundaries meet, in one lane's own candidates when `split`) are decided by
-// nearest64, so the boundary value is the one the per-thread query picks.
+// Whether two equally near primitives must be told apart as the reference's
+// traversal does: their closest points are not one point (a shared vertex or
+// edge, found through either, differs by ulps), or their boundaries differ.
+// Grid points on a symmetry plane of a box, say, are as far from its top as
+// from its bottom.
+template <int DIM>
+__device__ __forceinline__ bool tie_matters(const SceneView &s, int a, int b, double dx, double dy,
+                                            double dz, float margin) {
+    const double tol = 1e-3 * static_cast<double>(margin);
+    if (dx * dx + dy * dy + (DIM == 3 ? dz * dz : 0.0) > tol * tol) return true;
+    return DIM == 2 && s.segid[a].x != s.segid[b].x;
+}
+
+// This lane's nearest primitive so far (slot -1: none), its squared distance
+// and closest point; `split`: another one ties with it in a way that matters.
+struct LaneNearest {
+    double d2, x, y, z;
+    int slot;
+    bool split;
+};
+
+// The winner among the lanes' primitives.  Equally near ones: the lowest
+// slot, or where the choice matters what nearest64 picks, so that boundary
+// points and values are the per-thread query's.
 template <int DIM>
 __device__ __forceinline__ int winning_slot(const SceneView &s, double px, double py, double pz,
-                                            double best, int slot, bool split) {
+                                            const LaneNearest &c, float margin) {
     constexpr unsigned kAll = 0xffffffffu;
-    const double m = warp_min_double(best);
-    const bool mine = slot >= 0 && best == m;
+    const double m = warp_min_double(c.d2);
+    const bool mine = c.slot >= 0 && c.d2 == m;
     const unsigned ties = __ballot_sync(kAll, mine);
     if (!ties) return -1;
-    int win = __shfl_sync(kAll, slot, __ffs(ties) - 1);
-    if ((ties & (ties - 1u)) || __any_sync(kAll, mine && split)) {
-        win = static_cast<int>(
-            __reduce_min_sync(kAll, mine ? static_cast<unsigned>(slot) : 0xffffffffu));
-        if constexpr (DIM == 2) {
-            const int bid = s.segid[win].x;
-            if (__any_sync(kAll, mine && (split || s.segid[slot].x != bid))) {
-                win = nearest64<2>(s, px, py, pz, __longlong_as_double(0x7ff0000000000000LL)).slot;
-            }
+    const int from = __ffs(static_cast<int>(ties)) - 1;
+    int win = __shfl_sync(kAll, c.slot, from);
+    if ((ties & (ties - 1u)) || __any_sync(kAll, mine && c.split)) {
+        const double dx = c.x - __shfl_sync(kAll, c.x, from);
+        const double dy = c.y - __shfl_sync(kAll, c.y, from);
+        const double dz = DIM == 3 ? c.z - __shfl_sync(kAll, c.z, from) : 0.0;
+        if (__any_sync(kAll, mine && (c.split || tie_matters<DIM>(s, c.slot, win, dx, dy, dz,
+                                                                  margin)))) {
+            return nearest64<DIM>(s, px, py, pz, __longlong_as_double(0x7ff0000000000000LL)).slot;
         }
+        win = static_cast<int>(
+            __reduce_min_sync(kAll, mine ? static_cast<unsigned>(c.slot) : 0xffffffffu));
     }
     return win;
 }
@@ -179,9 +200,7 @@ __device__ __forceinline__ int warp_nearest64_full(const SceneView &s, const Wid
                                                    float margin) {
     constexpr unsigned kAll = 0xffffffffu;
     const int lane = static_cast<int>(threadIdx.x & 31u);
-    double best = __longlong_as_double(0x7ff0000000000000LL);
-    int slot = -1;
-    bool split = false;  // this lane saw a tie across two boundaries
+    LaneNearest c{__longlong_as_double(0x7ff0000000000000LL), 0.0, 0.0, 0.0, -1, false};
     float limit = INFINITY, ubest = INFINITY;
     visit_clusters<DIM>(w, static_cast<float>(px), static_cast<float>(py),
                         static_cast<float>(pz), limit, [&](int cluster) {
@@ -191,12 +210,12 @@ __device__ __forceinline__ int warp_nearest64_full(const SceneView &s, const Wid
             const int k = __ldg(w.wide2bin + ws);
             double nx, ny, nz;
             d2 = slot_dist64<DIM>(s, k, px, py, pz, nx, ny, nz);
-            if (DIM == 2 && d2 == best && s.segid[k].x != s.segid[slot].x) split = true;
-            if (d2 < best || (d2 == best && k < slot)) {
-                if (d2 < best) split = false;
-                best = d2;
-                slot = k;
-            }
+            const bool tie = d2 == c.d2 && c.slot >= 0;
+            const bool split =
+                tie && (c.split || tie_matters<DIM>(s, k, c.slot, nx - c.x, ny - c.y,
+                                                    DIM == 3 ? nz - c.z : 0.0, margin));
+            if (d2 < c.d2 || (tie && k < c.slot)) c = LaneNearest{d2, nx, ny, nz, k, split};
+            if (tie) c.split = split;
         }
         const float u = __uint_as_float(
             __reduce_min_sync(kAll, __float_as_uint(__double2float_ru(d2))));
@@ -205,7 +224,7 @@ __device__ __forceinline__ int warp_nearest64_full(const SceneView &s, const Wid
             limit = candidate_limit(u, margin);
         }
     });
-    return winning_slot<DIM>(s, px, py, pz, best, slot, split);
+    return winning_slot<DIM>(s, px, py, pz, c, margin);
 }
 
 // The primitives that can be nearest to a point: binary slots a and, when
@@ -297,27 +316,29 @@ __device__ __forceinline__ Candidates warp_candidates64(const SceneView &s, cons
     const int a = __shfl_sync(kAll, k, __ffs(near) - 1);
     if (rest == 0u) return Candidates{a, -1};
     if ((rest & (rest - 1u)) == 0u) return Candidates{a, __shfl_sync(kAll, k, __ffs(rest) - 1)};
-    double best = __longlong_as_double(0x7ff0000000000000LL);
-    const bool mine = (near >> lane) & 1u;
-    double nx, ny, nz;
-    if (mine) best = slot_dist64<DIM>(s, k, px, py, pz, nx, ny, nz);
-    return Candidates{winning_slot<DIM>(s, px, py, pz, best, mine ? k : -1, false), -1};
+    LaneNearest c{__longlong_as_double(0x7ff0000000000000LL), 0.0, 0.0, 0.0, -1, false};
+    if ((near >> lane) & 1u) {
+        c.slot = k;
+        c.d2 = slot_dist64<DIM>(s, k, px, py, pz, c.x, c.y, c.z);
+    }
+    return Candidates{winning_slot<DIM>(s, px, py, pz, c, margin), -1};
 }
 
 // The nearest of a point's candidates: its squared FP64 distance, closest
 // point and binary slot.  Equally near: as winning_slot decides.
 template <int DIM>
-__device__ __forceinline__ double pick_nearest64(const SceneView &s, Candidates c, double px,
-                                                 double py, double pz, int &slot, double &nx,
-                                                 double &ny, double &nz) {
+__device__ __forceinline__ double pick_nearest64(const SceneView &s, float margin, Candidates c,
+                                                 double px, double py, double pz, int &slot,
+                                                 double &nx, double &ny, double &nz) {
     slot = c.a;
     double d2 = slot_dist64<DIM>(s, c.a, px, py, pz, nx, ny, nz);
     if (c.b >= 0) {
         double bx, by, bz;
         const double e2 = slot_dist64<DIM>(s, c.b, px, py, pz, bx, by, bz);
         bool second = e2 < d2 || (e2 == d2 && c.b < c.a);
-        if (DIM == 2 && e2 == d2 && s.segid[c.a].x != s.segid[c.b].x) {
-            second = nearest64<2>(s, px, py, pz, __longlong_as_double(0x7ff0000000000000LL))
+        if (e2 == d2 && tie_matters<DIM>(s, c.a, c.b, bx - nx, by - ny,
+                                         DIM == 3 ? bz - nz : 0.0, margin)) {
+            second = nearest64<DIM>(s, px, py, pz, __longlong_as_double(0x7ff0000000000000LL))
                          .slot == c.b;
         }
         if (second) {
@@ -329,6 +350,129 @@ __device__ __forceinline__ double pick_nearest64(const SceneView &s, Candidates 
         }
     }
     return d2;
+}
+
+// Winding numbers of the mesh around G points, the segments spread over the
+// lanes (winding_number's sum, in any order); a segment is read once for all
+// G points.
+template <int G>
+struct WindingPoints {
+    double x[G], y[G];
+    int wn[G];
+};
+template <int G>
+__device__ __forceinline__ void warp_winding_numbers(const SceneView &s, WindingPoints<G> &q) {
+    const int lane = static_cast<int>(threadIdx.x & 31u);
+#pragma unroll
+    for (int g = 0; g < G; ++g) q.wn[g] = 0;
+    for (int k = lane; k < s.n_prims; k += 32) {
+        const double2 a = s.seg64[2 * k], c = s.seg64[2 * k + 1];
+#pragma unroll
+        for (int g = 0; g < G; ++g) {
+            const double area =
+                (c.x - a.x) * (q.y[g] - a.y) - (q.x[g] - a.x) * (c.y - a.y);
+            if (a.y <= q.y[g]) {
+                if (c.y > q.y[g] && area > 0) ++q.wn[g];
+            } else {
+                if (c.y <= q.y[g] && area < 0) --q.wn[g];
+            }
+        }
+    }
+#pragma unroll
+    for (int g = 0; g < G; ++g) q.wn[g] = __reduce_add_sync(0xffffffffu, q.wn[g]);
+}
+
+// Whether the ray meets the padded box of every node from the root to the
+// leaf of binary slot k, i.e. whether count_ray_hits tests that triangle.
+__device__ __forceinline__ bool ray_reaches(const SceneView &s, const double *p,
+                                            const double *ray, int k) {
+    int j = static_cast<int>(((static_cast<long long>(k) + 1) * (1ll << s.depth) - 1) / s.n_prims);
+    while (leaf_first(j, s.n_prims, s.depth) > k) --j;
+    while (leaf_first(j + 1, s.n_prims, s.depth) <= k) ++j;
+    for (unsigned id = (1u << s.depth) + static_cast<unsigned>(j); id >= 1u; id >>= 1) {
+        if (!ray_box(s.box64 + 6 * id, p, ray)) return false;
+    }
+    return true;
+}
+
+// count_ray_hits by the whole warp: FP32 tests of the wide tree's boxes,
+// padded by `pad` for their rounding, choose the leaf clusters, and the lanes
+// test a cluster's triangles in FP64.  A triangle that is crossed plainly is
+// one whose boxes the ray meets; one met at a grazing angle or ambiguously is
+// counted only if the reference's traversal reaches it (ray_reaches).
+__device__ __forceinline__ int warp_ray_hits(const SceneView &s, const WideView &w,
+                                             const double *p, const double *ray, float pad,
+                                             bool &ambiguous) {
+    constexpr unsigned kAll = 0xffffffffu;
+    const unsigned lane = threadIdx.x & 31u;
+    float o[3], inv[3];
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        o[k] = static_cast<float>(p[k]);
+        inv[k] = 1.0f / static_cast<float>(ray[k]);
+    }
+    auto meets = [&](int h, int parent) -> bool {
+        const float *b = w.box + w.off[h] + parent * (11 * 32) + lane;
+        float t0 = 0.0f, t1 = INFINITY;
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            const float lo = b[32 * k] - pad - o[k], hi = b[32 * (3 + k)] + pad - o[k];
+            // a ray along the slab (1 / 0): fminf and fmaxf pass over the NaN
+            // of 0 * inf, and an origin off the slab gives an empty interval
+            const float ta = lo * inv[k], tb = hi * inv[k];
+            t0 = fmaxf(t0, fminf(ta, tb));
+            t1 = fminf(t1, fmaxf(ta, tb));
+        }
+        // (padding children have lo = inf, hi = -inf)
+        return t0 <= t1 * (1.0f + 0x1p-20f) && b[0] < INFINITY;
+    };
+    int hits = 0;
+    ambiguous = false;
+    auto leaf = [&](int cluster) -> bool {
+        const int ws = cluster * 32 + static_cast<int>(lane);
+        int h = kMiss;
+        if (ws < w.n) {
+            const int k = __ldg(w.wide2bin + ws);
+            bool grazing;
+            h = moller_trumbore(p, ray, s.tri64 + 7 * k, grazing);
+            if ((h == kAmbiguous || (h == kHit && grazing)) && !ray_reaches(s, p, ray, k)) {
+                h = kMiss;
+            }
+        }
+        if (__any_sync(kAll, h == kAmbiguous)) return true;
+        hits += __popc(__ballot_sync(kAll, h == kHit));
+        return false;
+    };
+    if (w.H == 1) {
+        ambiguous = leaf(0);
+        return hits;
+    }
+    // mask[h]: children of height h (of the node parent[h]) still to visit
+    unsigned mask[8];
+    int parent[8];
+    int h = w.H - 1;
+    parent[h] = 0;
+    mask[h] = __ballot_sync(kAll, meets(h, 0));
+    for (;;) {
+        if (mask[h] == 0u) {
+            if (h == w.H - 1) return hits;
+            ++h;
+            continue;
+        }
+        const int k = __ffs(static_cast<int>(mask[h])) - 1;
+        mask[h] &= mask[h] - 1u;
+        const int child = parent[h] * 32 + k;
+        if (h == 1) {
+            if (leaf(child)) {
+                ambiguous = true;
+                return hits;
+            }
+        } else {
+            --h;
+            parent[h] = child;
+            mask[h] = __ballot_sync(kAll, meets(h, child));
+        }
+    }
 }
 
 }  // namespace wosb

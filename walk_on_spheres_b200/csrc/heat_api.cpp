@@ -39,7 +39,7 @@ int wos_context::run_heat(const wos_params &p, const HeatDesc &h, const PointSet
     const Fields cls{nullptr, nullptr, nullptr, nullptr, out.f.location};
 
     WOS_CUDA(this, cudaEventRecord(events[0], stream), "event");
-    WOS_CUDA(this, launch_classify(view, ps, p.seed, p.max_ray_attempts, btol, eq, cls, loc, st,
+    WOS_CUDA(this, launch_classify(view, wide, ps, p.seed, p.max_ray_attempts, btol, eq, cls, loc, st,
                                    ctr, stream),
              "classification kernel");
     WOS_CUDA(this, cudaEventRecord(events[1], stream), "event");

@@ -43,9 +43,9 @@ struct FastStart {
 // Start points, classification and boundary values for every point of `ps`
 // (include/wos/runner.hpp:170-206).  Writes location, start records and the
 // fields of non-inside points.
-cudaError_t launch_classify(const SceneView &s, const PointSet &ps, uint64_t seed,
-                            int max_ray_attempts, double boundary_tolerance, EqDesc eq,
-                            Fields out, uint8_t *location, StartRecord *start,
+cudaError_t launch_classify(const SceneView &s, const WideView &w, const PointSet &ps,
+                            uint64_t seed, int max_ray_attempts, double boundary_tolerance,
+                            EqDesc eq, Fields out, uint8_t *location, StartRecord *start,
                             DeviceCounters *counters, cudaStream_t stream,
                             const FastStart &fast = FastStart{});
 

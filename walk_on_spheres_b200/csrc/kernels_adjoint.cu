@@ -676,7 +676,7 @@ __device__ __forceinline__ void heat_task64(const HeatArgs &a, const WideView &w
                 if (lane == jl) cand = found;
             }
             if (query) {
-                R = sqrt(pick_nearest64<DIM>(a.s, cand, p.x, p.y, p.z, slot, np.x, np.y, np.z));
+                R = sqrt(pick_nearest64<DIM>(a.s, wv.margin64, cand, p.x, p.y, p.z, slot, np.x, np.y, np.z));
             }
         } else if (query) {
             const Nearest<double> q = nearest64<DIM>(a.s, p.x, p.y, p.z, dinf());

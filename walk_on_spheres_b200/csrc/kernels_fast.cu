@@ -506,7 +506,7 @@ __device__ __forceinline__ void fast_task64(const FastArgs a, const WideView &wv
             }
             if (query) {
                 int slot;
-                R = sqrt(pick_nearest64<DIM>(a.s, cand, p.x, p.y, p.z, slot, np.x, np.y, np.z));
+                R = sqrt(pick_nearest64<DIM>(a.s, wv.margin64, cand, p.x, p.y, p.z, slot, np.x, np.y, np.z));
                 bid = bid_of<DIM>(a.s, slot);
             }
         } else if (query) {
@@ -558,7 +558,7 @@ constexpr int pool_words() {
     return WalkPool<DIM, Eq, HC>::kFields * kPool + 8 * 32;
 }
 
-// Blocks per SM of the FP32 walk kernels: 4 (64 registers) for the height <= 3
+// Blocks per SM of the FP32 walk kernels: 4 (64 registers) for the height <= 4
 // traversals (5 spill: disk 7.2 -> 8.6 ms); 3 for the generic and lane-scan
 // ones and for equations with a rejection sampler, whose state would spill
 // (star of 777 segments, screened, Green: 3.89 -> 3.78 ms, uniform 2.65 -> 2.35).

@@ -137,7 +137,7 @@ extern "C" int wos_solve_grid_device_noalloc(wos_context *ctx, const wos_params 
         fs.exact_below = std::max(eps, btol);
         fs.margin = wosb::fp32_distance_margin(ctx->scene.bbox, ctx->scene.dim);
     }
-    e = wosb::launch_classify(ctx->view, ps, p->seed, p->max_ray_attempts, btol, eq, out, loc,
+    e = wosb::launch_classify(ctx->view, ctx->wide, ps, p->seed, p->max_ray_attempts, btol, eq, out, loc,
                               start, ctr, s, fs);
     if (e != cudaSuccess) return fail(ctx, WOS_ERR_CUDA, std::string("classification kernel: ") + cudaGetErrorString(e));
     cudaEventRecord(ctx->events[1], s);

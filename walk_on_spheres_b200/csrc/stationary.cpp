@@ -198,7 +198,7 @@ extern "C" int wos_stationary_solve(wos_context *ctx, const wos_stationary_param
     const double btol = 1e-10 * plate.scale;
     const EqDesc eq{kPlate, p.source_mode, 0.0, nullptr, &desc};
     const uint64_t seed = p.seed ^ p.case_stream;
-    WOS_CUDA(ctx, launch_classify(dev.view, ps, seed, 12, btol, eq,
+    WOS_CUDA(ctx, launch_classify(dev.view, dev.wide, ps, seed, 12, btol, eq,
                                   Fields{nullptr, nullptr, nullptr, nullptr, nullptr}, loc, st,
                                   ctr + 1, stream),
              "classification kernel");

@@ -269,7 +269,7 @@ extern "C" int wos_transient_solve(wos_context *ctx, const wos_transient_params 
     // plate-edge grid point is a boundary point with value 0
     const double btol = 1e-10 * plate.scale;
     const EqDesc cls_eq{kTransient, kGreen, alpha, nullptr};
-    WOS_CUDA(ctx, launch_classify(dev.view, ps, p.seed, 12, btol, cls_eq,
+    WOS_CUDA(ctx, launch_classify(dev.view, dev.wide, ps, p.seed, 12, btol, cls_eq,
                                   Fields{nullptr, nullptr, nullptr, nullptr, nullptr}, loc, st,
                                   ctr + steps, stream),
              "classification kernel");
