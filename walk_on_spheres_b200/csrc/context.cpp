@@ -66,6 +66,7 @@ cudaError_t DeviceBuffer::reserve(size_t n) {
 wos_context::~wos_context() {
     for (DeviceBuffer *b : all_buffers()) b->release();
     sdev.release();
+    if (staging) cudaFreeHost(staging);
     for (auto &ev : events) {
         if (ev) cudaEventDestroy(ev);
     }
@@ -73,8 +74,7 @@ wos_context::~wos_context() {
 }
 
 std::vector<DeviceBuffer *> wos_context::all_buffers() {
-    return {&location, &start,
-            &f_mean, &f_var, &f_se, &f_steps, &f_loc, &partials, &queue, &counters, &points,
+    return {&location, &start, &packed, &partials, &queue, &points,
             &index, &scratch_a, &scratch_b, &scratch_c, &scratch_d, &h_values, &h_gradu,
             &h_gradg, &h_grads, &h_jac, &h_jacse};
 }
@@ -490,15 +490,49 @@ std::string wosb::check_params(const wos_context *ctx, const wos_params *p) {
     return std::string();
 }
 
+int wos_context::finish_solve(DeviceCounters &hc, const HostFields *host, bool &fetched) {
+    static_assert(sizeof(DeviceCounters) <= kHeader, "the counters fit their header");
+    const size_t n = host ? static_cast<size_t>(host->n) : 0;
+    const size_t bytes = kHeader + n * (4 * sizeof(double) + 1);
+    fetched = host != nullptr && bytes <= kStaging;
+    if (!fetched) {
+        WOS_CUDA(this, cudaMemcpyAsync(&hc, packed.ptr, sizeof(hc), cudaMemcpyDeviceToHost,
+                                       stream), "read counters");
+        WOS_CUDA(this, cudaStreamSynchronize(stream), "solve");
+        return WOS_OK;
+    }
+    if (bytes > staging_bytes) {
+        // grown in steps of 64 KB up to kStaging, kept for the context's solves
+        const size_t want = (bytes + 65535) / 65536 * 65536;
+        if (staging) cudaFreeHost(staging);
+        staging = nullptr;
+        staging_bytes = 0;
+        WOS_CUDA(this, cudaMallocHost(&staging, want), "staging block");
+        staging_bytes = want;
+    }
+    WOS_CUDA(this, cudaMemcpyAsync(staging, packed.ptr, bytes, cudaMemcpyDeviceToHost, stream),
+             "read results");
+    WOS_CUDA(this, cudaStreamSynchronize(stream), "solve");
+    std::memcpy(&hc, staging, sizeof(hc));
+    if (hc.error_flags) return WOS_OK;  // the caller reports; nothing is handed out
+    const char *at = static_cast<const char *>(staging) + kHeader;
+    for (double *to : {host->mean, host->variance, host->se, host->steps}) {
+        if (to) std::memcpy(to, at, sizeof(double) * n);
+        at += sizeof(double) * n;
+    }
+    if (host->loc) std::memcpy(host->loc, at, n);
+    return WOS_OK;
+}
+
 int wos_context::run(const wos_params &p, const PointSet &ps, Fields out,
-                     wos_counters *counters_out) {
+                     wos_counters *counters_out, const HostFields *host) {
     cudaSetDevice(device);
     const long long n = ps.n;
     const int dim = scene.dim;
     WOS_CUDA(this, location.reserve(std::max<long long>(n, 1)), "alloc location");
     WOS_CUDA(this, start.reserve(sizeof(StartRecord) * std::max<long long>(n, 1)), "alloc start");
-    WOS_CUDA(this, counters.reserve(sizeof(DeviceCounters)), "alloc counters");
-    WOS_CUDA(this, cudaMemsetAsync(counters.ptr, 0, sizeof(DeviceCounters), stream),
+    WOS_CUDA(this, packed.reserve(kHeader), "alloc counters");
+    WOS_CUDA(this, cudaMemsetAsync(packed.ptr, 0, sizeof(DeviceCounters), stream),
              "clear counters");
 
     EqDesc eq{p.equation, p.source_mode, p.alpha, nullptr};
@@ -513,7 +547,7 @@ int wos_context::run(const wos_params &p, const PointSet &ps, Fields out,
     }
     auto *loc = static_cast<uint8_t *>(location.ptr);
     auto *st = static_cast<StartRecord *>(start.ptr);
-    auto *ctr = static_cast<DeviceCounters *>(counters.ptr);
+    auto *ctr = static_cast<DeviceCounters *>(packed.ptr);
 
     WOS_CUDA(this, cudaEventRecord(events[0], stream), "event");
     FastStart fs;
@@ -553,9 +587,8 @@ int wos_context::run(const wos_params &p, const PointSet &ps, Fields out,
     if (p.method == WOS_METHOD_PLAIN_FP64) WOS_CUDA(this, cudaEventRecord(events[2], stream), "event");
     WOS_CUDA(this, cudaEventRecord(events[3], stream), "event");
     DeviceCounters hc{};
-    WOS_CUDA(this, cudaMemcpyAsync(&hc, ctr, sizeof(hc), cudaMemcpyDeviceToHost, stream),
-             "read counters");
-    WOS_CUDA(this, cudaStreamSynchronize(stream), "solve");
+    bool fetched = false;
+    if (const int rc = finish_solve(hc, host, fetched)) return rc;
     if (hc.error_flags) return fail(this, WOS_ERR_DEVICE, device_error(hc.error_flags));
     if (counters_out) {
         wos_counters &c = *counters_out;
@@ -573,7 +606,7 @@ int wos_context::run(const wos_params &p, const PointSet &ps, Fields out,
         cudaEventElapsedTime(&c.total_ms, events[0], events[3]);
     }
     (void)dim;
-    return WOS_OK;
+    return host && !fetched ? download(out, *host) : WOS_OK;
 }
 
 PointSet wosb::grid_points(int dim, const wos_grid &g) {
@@ -616,25 +649,21 @@ extern "C" int wos_solve_grid_device(wos_context *ctx, const wos_params *params,
 }
 
 int wos_context::fields_for(long long n, Fields &out) {
-    WOS_CUDA(this, f_mean.reserve(sizeof(double) * std::max<long long>(n, 1)), "alloc mean");
-    WOS_CUDA(this, f_var.reserve(sizeof(double) * std::max<long long>(n, 1)), "alloc variance");
-    WOS_CUDA(this, f_se.reserve(sizeof(double) * std::max<long long>(n, 1)), "alloc se");
-    WOS_CUDA(this, f_steps.reserve(sizeof(double) * std::max<long long>(n, 1)), "alloc steps");
-    WOS_CUDA(this, f_loc.reserve(std::max<long long>(n, 1)), "alloc location");
-    out = Fields{static_cast<double *>(f_mean.ptr), static_cast<double *>(f_var.ptr),
-                 static_cast<double *>(f_se.ptr), static_cast<double *>(f_steps.ptr),
-                 static_cast<uint8_t *>(f_loc.ptr)};
+    const size_t m = static_cast<size_t>(std::max<long long>(n, 1));
+    WOS_CUDA(this, packed.reserve(kHeader + m * (4 * sizeof(double) + 1)), "alloc results");
+    auto *f = reinterpret_cast<double *>(static_cast<char *>(packed.ptr) + kHeader);
+    const size_t k = static_cast<size_t>(n);
+    out = Fields{f, f + k, f + 2 * k, f + 3 * k, reinterpret_cast<uint8_t *>(f + 4 * k)};
     return WOS_OK;
 }
 
-int wos_context::download(long long n, const Fields &dev, double *mean, double *variance,
-                          double *se, double *steps, uint8_t *loc) {
-    const size_t b = sizeof(double) * static_cast<size_t>(n);
-    if (mean) WOS_CUDA(this, cudaMemcpyAsync(mean, dev.mean, b, cudaMemcpyDeviceToHost, stream), "D2H");
-    if (variance) WOS_CUDA(this, cudaMemcpyAsync(variance, dev.variance, b, cudaMemcpyDeviceToHost, stream), "D2H");
-    if (se) WOS_CUDA(this, cudaMemcpyAsync(se, dev.standard_error, b, cudaMemcpyDeviceToHost, stream), "D2H");
-    if (steps) WOS_CUDA(this, cudaMemcpyAsync(steps, dev.mean_steps, b, cudaMemcpyDeviceToHost, stream), "D2H");
-    if (loc) WOS_CUDA(this, cudaMemcpyAsync(loc, dev.location, static_cast<size_t>(n), cudaMemcpyDeviceToHost, stream), "D2H");
+int wos_context::download(const Fields &dev, const HostFields &h) {
+    const size_t b = sizeof(double) * static_cast<size_t>(h.n);
+    if (h.mean) WOS_CUDA(this, cudaMemcpyAsync(h.mean, dev.mean, b, cudaMemcpyDeviceToHost, stream), "D2H");
+    if (h.variance) WOS_CUDA(this, cudaMemcpyAsync(h.variance, dev.variance, b, cudaMemcpyDeviceToHost, stream), "D2H");
+    if (h.se) WOS_CUDA(this, cudaMemcpyAsync(h.se, dev.standard_error, b, cudaMemcpyDeviceToHost, stream), "D2H");
+    if (h.steps) WOS_CUDA(this, cudaMemcpyAsync(h.steps, dev.mean_steps, b, cudaMemcpyDeviceToHost, stream), "D2H");
+    if (h.loc) WOS_CUDA(this, cudaMemcpyAsync(h.loc, dev.location, static_cast<size_t>(h.n), cudaMemcpyDeviceToHost, stream), "D2H");
     WOS_CUDA(this, cudaStreamSynchronize(stream), "D2H");
     return WOS_OK;
 }
@@ -670,8 +699,6 @@ extern "C" int wos_solve_grid(wos_context *ctx, const wos_params *params, const 
     Fields dev{};
     int rc = ctx->fields_for(ps.n, dev);
     if (rc) return rc;
-    rc = ctx->run(*params, ps, dev, counters);
-    if (rc) return rc;
     // the diagnostics need the location and statistics even when the caller
     // skips them
     std::vector<double> tv, ts, tst;
@@ -684,7 +711,8 @@ extern "C" int wos_solve_grid(wos_context *ctx, const wos_params *params, const 
         if (!m) { tst.resize(ps.n); m = tst.data(); }
         if (!l) { tl.resize(ps.n); l = tl.data(); }
     }
-    rc = ctx->download(ps.n, dev, mean, v, s, m, l);
+    const wos_context::HostFields host{ps.n, mean, v, s, m, l};
+    rc = ctx->run(*params, ps, dev, counters, &host);
     if (rc) return rc;
     host_sums(ps.n, v, s, m, l, counters);
     return WOS_OK;
@@ -727,9 +755,8 @@ extern "C" int wos_solve_points(wos_context *ctx, const wos_params *params, cons
     Fields dev{};
     int rc = ctx->fields_for(n, dev);
     if (rc) return rc;
-    rc = ctx->run(*params, ps, dev, counters);
-    if (rc) return rc;
-    return ctx->download(n, dev, mean, variance, standard_error, mean_steps, location);
+    const wos_context::HostFields host{n, mean, variance, standard_error, mean_steps, location};
+    return ctx->run(*params, ps, dev, counters, &host);
 }
 
 // ------------------------------------------------------------- checks

@@ -127,8 +127,15 @@ struct wos_context {
     // scene
     wosb::SceneDevice sdev;
     // per solve
-    wosb::DeviceBuffer location, start, f_mean, f_var, f_se, f_steps, f_loc, partials, queue,
-        counters, points, index;
+    wosb::DeviceBuffer location, start, partials, queue, points, index;
+    // the solve's counters (kHeader bytes), then the host entry points' result
+    // fields end to end, so a small result comes back in one copy
+    static constexpr size_t kHeader = 256;
+    wosb::DeviceBuffer packed;
+    // page-locked landing place of such a copy: at most kStaging bytes
+    static constexpr size_t kStaging = size_t(1) << 20;
+    void *staging = nullptr;
+    size_t staging_bytes = 0;
     // kernel-level checks
     wosb::DeviceBuffer scratch_a, scratch_b, scratch_c, scratch_d;
     // Gaussian heat source: vertex values, probe weights, gradients, Jacobian
@@ -148,11 +155,20 @@ struct wos_context {
     ~wos_context();
     std::vector<wosb::DeviceBuffer *> all_buffers();
     int upload_scene();
-    int run(const wos_params &p, const wosb::PointSet &ps, wosb::Fields out, wos_counters *c);
+    // Host arrays (any may be null) that the fields of fields_for(n) go to.
+    struct HostFields {
+        long long n;
+        double *mean, *variance, *se, *steps;
+        uint8_t *loc;
+    };
+    int run(const wos_params &p, const wosb::PointSet &ps, wosb::Fields out, wos_counters *c,
+            const HostFields *host = nullptr);
     // Heat-source forward (h.adjoint == 0) or adjoint replay over `ps`.
     int run_heat(const wos_params &p, const wosb::HeatDesc &h, const wosb::PointSet &ps,
                  wosb::HeatOut out, wos_counters *c);
     int fields_for(long long n, wosb::Fields &out);
-    int download(long long n, const wosb::Fields &dev, double *mean, double *variance, double *se,
-                 double *steps, uint8_t *loc);
+    int download(const wosb::Fields &dev, const HostFields &host);
+    // The counters and, when they fit the staging block, the fields of `host`
+    // (`fetched` tells) after everything queued; waits for the stream.
+    int finish_solve(wosb::DeviceCounters &hc, const HostFields *host, bool &fetched);
 };

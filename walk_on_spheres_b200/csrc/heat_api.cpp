@@ -26,12 +26,12 @@ int wos_context::run_heat(const wos_params &p, const HeatDesc &h, const PointSet
     }
     WOS_CUDA(this, location.reserve(std::max<long long>(n, 1)), "alloc location");
     WOS_CUDA(this, start.reserve(sizeof(StartRecord) * std::max<long long>(n, 1)), "alloc start");
-    WOS_CUDA(this, counters.reserve(sizeof(DeviceCounters)), "alloc counters");
-    WOS_CUDA(this, cudaMemsetAsync(counters.ptr, 0, sizeof(DeviceCounters), stream),
+    WOS_CUDA(this, packed.reserve(kHeader), "alloc counters");
+    WOS_CUDA(this, cudaMemsetAsync(packed.ptr, 0, sizeof(DeviceCounters), stream),
              "clear counters");
     auto *loc = static_cast<uint8_t *>(location.ptr);
     auto *st = static_cast<StartRecord *>(start.ptr);
-    auto *ctr = static_cast<DeviceCounters *>(counters.ptr);
+    auto *ctr = static_cast<DeviceCounters *>(packed.ptr);
     // boundary tolerance 1e-10 * max(1, mesh extents), include/wos/runner.hpp:86-88
     const double btol = 1e-10 * scene.scale;
     // classification only: the heat merge writes every field
@@ -208,7 +208,7 @@ extern "C" int wos_heat_forward(wos_context *ctx, const wos_params *params,
     HeatOut out{dev, nullptr, nullptr, nullptr};
     rc = ctx->run_heat(*params, h, ps, out, counters);
     if (rc) return rc;
-    return ctx->download(n, dev, mean, variance, standard_error, mean_steps, location);
+    return ctx->download(dev, {n, mean, variance, standard_error, mean_steps, location});
 }
 
 extern "C" int wos_heat_adjoint(wos_context *ctx, const wos_params *params,
