@@ -106,6 +106,37 @@ __device__ __forceinline__ V3<T> sphere_step(V3<T> c, T R, Rng &rng) {
     }
 }
 
+// The direction of a step, drawn ahead of it (PLAIN_FP64): 2D cos and sin of
+// the angle, 3D also the height z and its circle's radius r.
+struct Direction {
+    double c, s, r, z;
+};
+
+// sphere_step with the draws already made, in the same expressions.
+template <int DIM, bool EXACT, typename T>
+__device__ __forceinline__ V3<T> sphere_step(V3<T> c, T R, const Direction &d) {
+    static_assert(EXACT, "the exact path's expressions");
+    if (DIM == 2) return V3<T>{c.x + R * d.c, c.y + R * d.s, T(0)};
+    return V3<T>{c.x + R * d.r * d.c, c.y + R * d.r * d.s, c.z + R * d.z};
+}
+
+// Draws the direction of sphere_step<DIM, true>.
+template <int DIM, class Rng>
+__device__ __forceinline__ void direction_draws(Rng &rng, double &u, double &v) {
+    u = rng.unit();
+    v = DIM == 3 ? rng.unit() : 0.0;
+}
+template <int DIM>
+__device__ __forceinline__ Direction direction_of(double u, double v) {
+    if (DIM == 2) {
+        const double theta = u * 2 * kPi;
+        return Direction{cos(theta), sin(theta), 1.0, 0.0};
+    }
+    const double z = 2.0 * u - 1.0;
+    const double phi = 2 * kPi * v;
+    return Direction{cos(phi), sin(phi), sqrt(1.0 - z * z), z};
+}
+
 // Uniform point in the ball, src/wos.cpp:33-56.
 template <int DIM, bool EXACT, typename T, class Rng>
 __device__ __forceinline__ V3<T> ball_sample(V3<T> c, T R, Rng &rng) {

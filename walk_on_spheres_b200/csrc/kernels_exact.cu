@@ -346,6 +346,32 @@ __global__ void __launch_bounds__(kExactThreads)
     }
 }
 
+// Stands in for source draws that were taken from the stream beforehand and
+// whose sample has no effect (3D sources are zero).
+struct SkippedDraws {
+    __device__ __forceinline__ double unit() { return 0.5; }
+    __device__ __forceinline__ double unit_open() { return 0.5; }
+};
+
+// Takes one step's draws from a point's walk stream: in 3D, where one stream
+// serves both, the source sample's first (six for a Green sample, three for a
+// uniform one), then the direction's.
+template <int DIM, class Eq>
+__device__ __forceinline__ void step_draws(const Eq &eq, Xoshiro &rng, double &u, double &v) {
+    if constexpr (DIM == 3 && Eq::kSource) {
+        if (eq.mode == kGreen) {
+            for (int k = 0; k < 4; ++k) rng.unit_open();
+            rng.unit();
+            rng.unit();
+        } else {
+            rng.unit();
+            rng.unit();
+            rng.unit_open();
+        }
+    }
+    direction_draws<DIM>(rng, u, v);
+}
+
 // The walks of one point, one step of the current walk at a time.  A point's
 // walks run one after another on its streams (where a walk's draws begin
 // depends on every walk before it), so the point is the unit of parallel work.
@@ -387,6 +413,17 @@ struct PlainWalks {
     }
     __device__ __forceinline__ bool stepping(double eps, int max_steps) const {
         return R > eps && steps < max_steps;
+    }
+    // A step whose direction was drawn ahead (draw_ahead); in 3D the source
+    // sample, whose draws were skipped then, is that of a zero source.
+    __device__ __forceinline__ void step(const Eq &eq, const Direction &d) {
+        if constexpr (DIM == 2) {
+            p = walk_body<2, true, double>(eq, p, R, sample, weight, d, src, overflow);
+        } else {
+            SkippedDraws none;
+            p = walk_body<3, true, double>(eq, p, R, sample, weight, d, none, overflow);
+        }
+        ++steps;
     }
     __device__ __forceinline__ void step(const Eq &eq) {
         if (DIM == 2) {
@@ -458,14 +495,18 @@ __global__ void __launch_bounds__(kExactThreads)
     }
 }
 
-// `per_warp` consecutive points per warp, one per lane; every iteration
-// steps each lane's walk and the whole warp then answers the lanes' queries
-// one after another (warp_candidates64).  A point's walks are serial, so the
-// kernel waits on one step's chain (draw, sine and cosine, query, square
-// root) rather than on issue slots.  Per-thread queries made that chain 30
-// dependent tree nodes long in 32 diverging lanes: 1360 inside points of an
-// annulus of 256 segments, 1000 walks, took 144.8 ms, now 10.4; 0.41 M walks
-// in a blob of 3968 triangles 425 ms, now 9.5 (same results, bit for bit).
+// `per_warp` consecutive points per warp, each owned by the first lane of its
+// group of 32 / per_warp lanes.  Every iteration steps each point's walk and
+// the whole warp then answers the points' queries one after another
+// (warp_candidates64).  A point's walks are serial, so the kernel waits on one
+// step's chain (draw, sine and cosine, query, square root) rather than on issue
+// slots.  Per-thread queries made that chain 30 dependent tree nodes long in 32
+// diverging lanes.  The draws do not depend on the walk, so a group takes its
+// point's next draws together, one step's per lane, and forms all their sines
+// and cosines at once (each lane keeps the stream and picks its own draws).
+// 1360 inside points of an annulus of 256 segments, 1000 walks: 144.8 ms by
+// threads, 10.4 by warps, 8.6 ms with directions drawn ahead; 0.41 M walks in a
+// blob of 3968 triangles 425, 9.4 and 8.9 ms (same results, bit for bit).
 template <int DIM, class Eq>
 __global__ void __launch_bounds__(kExactThreads, 4)
     walk_plain_warp_kernel(SceneView s, WideView w, int per_warp, PointSet ps, uint64_t seed,
@@ -479,14 +520,46 @@ __global__ void __launch_bounds__(kExactThreads, 4)
     __syncthreads();
     w.off = s_off;
     const int lane = threadIdx.x & 31;
+    const int group = 32 / per_warp, sub = lane % group;
     const long long warp = (static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
-    const long long t = warp * per_warp + lane;
-    bool active = lane < per_warp && t < ps.n && location[t] == 1;
+    const long long t = warp * per_warp + lane / group;
+    const bool mine = t < ps.n && location[t] == 1;  // the group has a point to walk
+    bool active = mine && sub == 0;
     if (!__any_sync(kAll, active)) return;
-    PlainWalks<DIM, Eq> k(ps, active ? t : 0, seed, start);
+    PlainWalks<DIM, Eq> k(ps, mine ? t : 0, seed, start);
+    Direction ahead{0.0, 0.0, 0.0, 0.0};  // the group's step `used` + sub
+    int used = group;                     // directions of the batch taken so far
     while (__any_sync(kAll, active)) {
         const bool query = active && k.stepping(eps, max_steps);
-        if (query) k.step(eq);
+        // groups whose batch is used up draw the next one
+        const bool refill =
+            __shfl_sync(kAll, static_cast<int>(query && used == group), lane - sub) != 0;
+        if (__any_sync(kAll, refill)) {
+            if (refill) {
+                double u = 0.0, v = 0.0;
+                for (int i = 0; i < group; ++i) {
+                    double ui, vi;
+                    step_draws<DIM>(eq, k.walk, ui, vi);
+                    if (i == sub) {
+                        u = ui;
+                        v = vi;
+                    }
+                }
+                ahead = direction_of<DIM>(u, v);
+                used = 0;
+            }
+            __syncwarp();
+        }
+        const int from = lane - sub + (query ? used : 0);
+        Direction d;
+        d.c = __shfl_sync(kAll, ahead.c, from);
+        d.s = __shfl_sync(kAll, ahead.s, from);
+        d.r = DIM == 3 ? __shfl_sync(kAll, ahead.r, from) : 1.0;
+        d.z = DIM == 3 ? __shfl_sync(kAll, ahead.z, from) : 0.0;
+        if (query) {
+            k.step(eq, d);
+            ++used;
+        }
         unsigned pending = __ballot_sync(kAll, query);
         Candidates cand{0, -1};
         while (pending) {
@@ -499,8 +572,8 @@ __global__ void __launch_bounds__(kExactThreads, 4)
         }
         if (query) {
             int slot;
-            k.R = sqrt(pick_nearest64<DIM>(s, w.margin64, cand, k.p.x, k.p.y, k.p.z, slot, k.np.x, k.np.y,
-                                           k.np.z));
+            k.R = sqrt(pick_nearest64<DIM>(s, w.margin64, cand, k.p.x, k.p.y, k.p.z, slot, k.np.x,
+                                           k.np.y, k.np.z));
             if (DIM == 2) k.bid = s.segid[slot].x;
         }
         if (active && !k.stepping(eps, max_steps)) {
@@ -551,14 +624,11 @@ int blocks_for(long long n, int threads) {
 // Points per warp of walk_plain_warp_kernel.  A warp answers its lanes'
 // queries in turn, so few points per warp give short steps, and many share
 // the cost of the step's arithmetic (one instruction stream for all lanes).
-// Measured on a B200, walk kernel in ms at 1 / 2 / 4 / 8 / 16 points per warp:
-// 2D circle of 1024 segments, 64 walks: 24^2 points 0.86 / 1.17 / 1.75 / 2.92
-// / 4.83; 64^2 1.50 / 1.28 / 1.94 / 3.14 / 5.36; 128^2 4.37 / 3.53 / 3.70 /
-// 3.57 / 5.66; 256^2 16.3 / 12.6 / 10.9 / 10.0 / 11.7.  3D sphere of 16 128
-// triangles, 16 walks (queries dominate the step): 24^3 3.88 / 4.15 / 4.37 /
-// 7.31 / 12.1; 40^3 15.4 / 14.4 / 14.7 / 16.5 / 18.3 (all with every query
-// compared in FP64; the rule's choices since: 0.82, 1.17, 2.93, 8.16; 3.18,
-// 11.0).
+// Measured on a B200, walk kernel in ms at 1 / 2 / 4 / 8 points per warp: 2D
+// circle of 1024 segments, 64 walks: 32^2 points 0.69 / 0.94 / 1.47 / 2.33; 64^2
+// 1.19 / 1.05 / 1.58 / 2.50; 128^2 3.46 / 2.86 / 2.99 / 2.86; 256^2 12.8 / 10.1 /
+// 8.71 / 7.89.  3D sphere of 16 128 triangles, 16 walks (queries dominate the
+// step): 24^3 3.08 / 3.10 / 3.08 / 5.06; 40^3 12.2 / 10.9 / 10.6 / 11.7.
 int points_per_warp(int dim, long long n) {
     if (dim == 3) return n >= 32768 ? 2 : 1;
     int p = 1;
