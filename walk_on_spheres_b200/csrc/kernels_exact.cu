@@ -637,8 +637,8 @@ int points_per_warp(int dim, long long n) {
 }
 
 template <int DIM, class Eq>
-void launch_plain_typed(const SceneView &s, const WideView &w, const PointSet &ps, uint64_t seed, const Eq &eq,
-                        int n_walks, double eps, int max_steps, const uint8_t *location,
+void launch_plain_typed(const SceneView &s, const WideView &w, const PointSet &ps, uint64_t seed,
+                        const Eq &eq, int n_walks, double eps, int max_steps, const uint8_t *location,
                         const StartRecord *start, Fields out, DeviceCounters *ctr,
                         cudaStream_t stream) {
     if (w.margin64 >= 0.0f) {
@@ -654,8 +654,8 @@ void launch_plain_typed(const SceneView &s, const WideView &w, const PointSet &p
 }
 
 template <int DIM>
-void launch_plain_dim(const SceneView &s, const WideView &w, const PointSet &ps, uint64_t seed, EqDesc e,
-                      int n_walks, double eps, int max_steps, const uint8_t *location,
+void launch_plain_dim(const SceneView &s, const WideView &w, const PointSet &ps, uint64_t seed,
+                      EqDesc e, int n_walks, double eps, int max_steps, const uint8_t *location,
                       const StartRecord *start, Fields out, DeviceCounters *ctr,
                       cudaStream_t stream) {
     switch (e.kind) {

@@ -2,12 +2,12 @@
 //
 // Scheduling.  A persistent grid of warps pulls tasks from a device queue
 // (one atomicAdd per task).  A task is a chunk of consecutive walks of one
-// grid point; its 32 lanes each run one walk at a time and, when a walk
-// ends, the lane is regenerated with the next walk index of the chunk
-// (warp ballot + popcount rank), so a warp stays full until the chunk's last
-// walks.  Every walk of point p with index w draws from its own Philox
-// stream keyed by p's reference seed, so results do not depend on which
-// lane or warp runs the walk.
+// grid point; its 32 lanes each run one walk at a time and take the next walk
+// index of the chunk when theirs ends (warp ballot + popcount rank) or, in
+// FAST_FP32, is put aside for a query (fast_task32), so a warp stays full
+// until the chunk's last walks.  Every walk of point p with index w draws from
+// its own Philox stream keyed by p's reference seed, so results do not depend
+// on which lane or warp runs the walk.
 //
 // Precision (FAST_FP32).  Positions, radii, closest-point queries and the
 // sphere step are FP32 against the FP32 scene (staged in shared memory when
