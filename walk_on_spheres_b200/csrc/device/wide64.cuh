@@ -331,6 +331,10 @@ __device__ __forceinline__ double pick_nearest64(const SceneView &s, float margi
                                                  double px, double py, double pz, int &slot,
                                                  double &nx, double &ny, double &nz) {
     slot = c.a;
+    if (c.a < 0) {  // no finite distance (a point too far away to square)
+        nx = ny = nz = 0.0;
+        return __longlong_as_double(0x7ff0000000000000LL);
+    }
     double d2 = slot_dist64<DIM>(s, c.a, px, py, pz, nx, ny, nz);
     if (c.b >= 0) {
         double bx, by, bz;

@@ -218,7 +218,7 @@ __device__ __forceinline__ StartRecord warp_start(const SceneView &s, const Wide
     const Candidates c = warp_candidates64<DIM>(s, w, p[0], p[1], z);
     st.radius = sqrt(
         pick_nearest64<DIM>(s, w.margin64, c, p[0], p[1], z, st.slot, st.nx, st.ny, st.nz));
-    st.boundary_id = DIM == 2 ? s.segid[st.slot].x : -1;
+    st.boundary_id = DIM == 2 && st.slot >= 0 ? s.segid[st.slot].x : -1;
     return st;
 }
 
@@ -574,7 +574,7 @@ __global__ void __launch_bounds__(kExactThreads, 4)
             int slot;
             k.R = sqrt(pick_nearest64<DIM>(s, w.margin64, cand, k.p.x, k.p.y, k.p.z, slot, k.np.x,
                                            k.np.y, k.np.z));
-            if (DIM == 2) k.bid = s.segid[slot].x;
+            if (DIM == 2) k.bid = slot >= 0 ? s.segid[slot].x : -1;
         }
         if (active && !k.stepping(eps, max_steps)) {
             k.end(eq, eps, start);
