@@ -1,0 +1,98 @@
+"""Points so far away that FP32 distances to the mesh overflow, or nearly do.
+
+Their queries stay on the per-thread FP64 tree.  The meshes have wide trees of
+one to four heights, because a node's padding children (at distance infinity)
+are what a query without any finite FP32 distance must not enter.  Far points
+lie outside; the points beside them keep the values of a solve without them,
+bit for bit (a point's streams depend on its own index).  Walks that leave an
+open surface take the same queries; their number that reaches the step cap is
+the oracle's to 5 binomial standard deviations (single walks are not compared:
+900 steps amplify rounding until they part).
+"""
+from __future__ import annotations
+
+import numpy as np
+import pytest
+
+from walk_on_spheres_b200 import meshes
+from walk_on_spheres_b200.heat import HeatProblem
+from walk_on_spheres_b200.meshes import Mesh
+
+pytestmark = pytest.mark.gpu
+
+MESHES = {
+    "height1_2d": lambda: meshes.circle(segments=30),
+    "height2_2d": lambda: meshes.circle(segments=300),
+    "height3_2d": lambda: meshes.circle(segments=1100),
+    "height4_2d": lambda: meshes.circle(segments=33000),
+    "height1_3d": lambda: meshes.uv_sphere(lon=5, lat=4),
+    "height2_3d": lambda: meshes.uv_sphere(lon=20, lat=11),
+    "height3_3d": lambda: meshes.uv_sphere(lon=40, lat=21),
+    "height4_3d": lambda: meshes.uv_sphere(lon=180, lat=95),
+}
+FAR = (1e8, 9.9e8, 1.01e9, 1e13, 1.8e19, 2e19, 1e20, 3e38, 4e38, 1e77, 1e155, 1e300)
+
+
+def _points(dim):
+    rng = np.random.default_rng(8)
+    near = rng.uniform(-0.3, 0.3, size=(9, dim))
+    far = [s * v * np.eye(dim)[k] for v in FAR for k in range(dim) for s in (1.0, -1.0)]
+    far += [np.full(dim, -v) for v in FAR]
+    return near, np.array(far)
+
+
+@pytest.mark.parametrize("method", ["fast", "fast64", "plain"])
+@pytest.mark.parametrize("name", MESHES)
+def test_far_points_are_outside(solver, name, method):
+    m = MESHES[name]()
+    solver.set_mesh(m)
+    near, far = _points(m.dim)
+    kw = dict(N_walks=16, seed=3, method=method)
+    alone = solver.solve_points("laplace", near, **kw)
+    both = solver.solve_points("laplace", np.concatenate([near, far]), **kw)
+    n = len(near)
+    assert alone.location.tolist() == [1] * n
+    assert both.location.tolist() == [1] * n + [0] * len(far)
+    assert np.isnan(both.mean[n:]).all()
+    assert np.array_equal(both.mean[:n], alone.mean)
+    assert np.array_equal(both.mean_steps[:n], alone.mean_steps)
+
+
+@pytest.mark.parametrize("method", ["fast", "fast64"])
+@pytest.mark.parametrize("name", ["height3_2d", "height4_3d"])
+def test_far_heat_probes_are_outside(solver, name, method):
+    m = MESHES[name]()
+    solver.set_mesh(m)
+    near, far = _points(m.dim)
+    theta = (1.0, (0.1,) * m.dim, 0.2)
+    g = np.linspace(-1.0, 1.0, len(m.verts))
+    kw = dict(N_walks=16, epsilon=1e-3, seed=3, method=method)
+    alone = HeatProblem(solver, near, **kw).forward(*theta, g)
+    both = HeatProblem(solver, np.concatenate([near, far]), **kw).forward(*theta, g)
+    n = len(near)
+    assert both.location.tolist() == [1] * n + [0] * len(far)
+    assert np.array_equal(both.mean[:n], alone.mean)
+
+
+def _open_sphere():
+    m = meshes.uv_sphere(lon=60, lat=31)
+    p = m.prims[m.verts[m.prims].mean(axis=1)[:, 2] > -0.1]
+    return Mesh(3, m.verts, p, np.zeros(len(p), dtype=np.int32))
+
+
+def test_walks_that_leave_an_open_surface(solver, oracle):
+    from oracle.oracle import Solve
+    m = _open_sphere()
+    assert len(m.prims) > 1024
+    solver.set_mesh(m)
+    kw = dict(N_walks=12, seed=7, max_steps=900)
+    ref = oracle.solve_grid("laplace", Solve(m, 7, 7, 7, **kw))
+    n = 12 * int((ref.location == 1).sum())
+    hits = ref.counters["max_steps_hits"]
+    assert 0.05 * n < hits < 0.95 * n
+    q = hits / n
+    for method in ("plain", "fast64"):
+        r = solver.solve_grid("laplace", 7, 7, 7, method=method, **kw)
+        assert np.array_equal(r.location, ref.location.reshape(r.location.shape))
+        assert np.isfinite(r.mean[r.location == 1]).all()
+        assert abs(r.counters["max_steps_hits"] - hits) <= 5.0 * np.sqrt(2.0 * n * q * (1.0 - q))

@@ -13,7 +13,8 @@
 // covers the rounding of the point to FP32 and of the bound arithmetic.  A
 // cluster is skipped only when its bound exceeds the best distance found plus
 // twice that margin.  wide64_usable() says for which scenes the margin is
-// meaningful; others keep the per-thread query.
+// meaningful; others keep the per-thread query, and so does a point too far
+// away for FP32 distances (fp32_reaches).
 #pragma once
 #include "scene.cuh"
 #include "wide.cuh"
@@ -32,6 +33,17 @@ inline bool wide64_usable(const double bbox[6], int dim, float margin) {
         mag = mag > (hi < 0 ? -hi : hi) ? mag : (hi < 0 ? -hi : hi);
     }
     return ext > 1e-9 && mag < 1e9 && static_cast<double>(margin) < 1e-3 * ext;
+}
+
+// Whether FP32 distances from p to such a scene are finite numbers: squares of
+// up to 2e9 and the triangle test's products of two of them stay below 3.4e38.
+// False for a NaN coordinate as well.
+__device__ __forceinline__ bool fp32_reaches(float px, float py, float pz) {
+    return fabsf(px) < 1e9f && fabsf(py) < 1e9f && fabsf(pz) < 1e9f;
+}
+// A traversal's first limit: none of the tree's nodes is below -1.
+__device__ __forceinline__ float first_limit(float px, float py, float pz) {
+    return fp32_reaches(px, py, pz) ? INFINITY : -1.0f;
 }
 
 // Up to this many primitives a lane's own FP64 query (nearest64) beats the
@@ -57,9 +69,11 @@ __device__ __forceinline__ double slot_dist64(const SceneView &s, int k, double 
                           r5.x, r5.y, r6.x, r6.y, nx, ny, nz);
 }
 
-// Visits the leaf clusters whose FP32 lower bound is at most `limit` (which
+// Visits the leaf clusters whose FP32 lower bound is below `limit` (which
 // leaf(cluster) lowers), nearest child first.  All 32 lanes call it with the
-// same point.
+// same point and `limit` at first_limit.  The comparisons are strict: infinity
+// is the distance of a node's padding children, which have no nodes or clusters
+// of their own, and (for a point that FP32 does not reach) of real ones.
 template <int DIM, class Leaf>
 __device__ __forceinline__ void visit_clusters(const WideView &w, float px, float py, float pz,
                                                const float &limit, Leaf &&leaf) {
@@ -77,10 +91,10 @@ __device__ __forceinline__ void visit_clusters(const WideView &w, float px, floa
     }
     if (w.H == 2) {
         const float d = wide_box_dist<DIM>(w, 1, 0, px, py, pz);
-        unsigned m = __ballot_sync(kAll, d <= limit);
+        unsigned m = __ballot_sync(kAll, d < limit);
         while (m) {
             leaf(take_nearest(m, d));
-            m &= __ballot_sync(kAll, d <= limit);
+            m &= __ballot_sync(kAll, d < limit);
         }
         return;
     }
@@ -91,18 +105,18 @@ __device__ __forceinline__ void visit_clusters(const WideView &w, float px, floa
     int h = w.H - 1;
     int node = 0;
     float top = wide_box_dist<DIM>(w, h, 0, px, py, pz);
-    unsigned m2 = __ballot_sync(kAll, top <= limit);
+    unsigned m2 = __ballot_sync(kAll, top < limit);
     for (;;) {
         if (h == 2) {
             while (m2) {
                 const int n2 = node * 32 + take_nearest(m2, top);
                 const float d1 = wide_box_dist<DIM>(w, 1, n2, px, py, pz);
-                unsigned m1 = __ballot_sync(kAll, d1 <= limit);
+                unsigned m1 = __ballot_sync(kAll, d1 < limit);
                 while (m1) {
                     leaf(n2 * 32 + take_nearest(m1, d1));
-                    m1 &= __ballot_sync(kAll, d1 <= limit);
+                    m1 &= __ballot_sync(kAll, d1 < limit);
                 }
-                m2 &= __ballot_sync(kAll, top <= limit);
+                m2 &= __ballot_sync(kAll, top < limit);
             }
         } else if (m2) {
             const int child = node * 32 + take_nearest(m2, top);
@@ -111,7 +125,7 @@ __device__ __forceinline__ void visit_clusters(const WideView &w, float px, floa
             node = child;
             --h;
             top = wide_box_dist<DIM>(w, h, node, px, py, pz);
-            m2 = __ballot_sync(kAll, top <= limit);
+            m2 = __ballot_sync(kAll, top < limit);
             continue;
         }
         // this node is done: back to its parent's pending children, whose
@@ -120,7 +134,7 @@ __device__ __forceinline__ void visit_clusters(const WideView &w, float px, floa
         ++h;
         node = parent[h];
         top = wide_box_dist<DIM>(w, h, node, px, py, pz);
-        m2 = mask[h] & __ballot_sync(kAll, top <= limit);
+        m2 = mask[h] & __ballot_sync(kAll, top < limit);
     }
 }
 
@@ -166,7 +180,8 @@ struct LaneNearest {
 
 // The winner among the lanes' primitives.  Equally near ones: the lowest
 // slot, or where the choice matters what nearest64 picks, so that boundary
-// points and values are the per-thread query's.
+// points and values are the per-thread query's.  Without any (a point that
+// FP32 does not reach) the per-thread query answers.
 template <int DIM>
 __device__ __forceinline__ int winning_slot(const SceneView &s, double px, double py, double pz,
                                             const LaneNearest &c, float margin) {
@@ -174,19 +189,23 @@ __device__ __forceinline__ int winning_slot(const SceneView &s, double px, doubl
     const double m = warp_min_double(c.d2);
     const bool mine = c.slot >= 0 && c.d2 == m;
     const unsigned ties = __ballot_sync(kAll, mine);
-    if (!ties) return -1;
-    const int from = __ffs(static_cast<int>(ties)) - 1;
-    int win = __shfl_sync(kAll, c.slot, from);
-    if ((ties & (ties - 1u)) || __any_sync(kAll, mine && c.split)) {
-        const double dx = c.x - __shfl_sync(kAll, c.x, from);
-        const double dy = c.y - __shfl_sync(kAll, c.y, from);
-        const double dz = DIM == 3 ? c.z - __shfl_sync(kAll, c.z, from) : 0.0;
-        if (__any_sync(kAll, mine && (c.split || tie_matters<DIM>(s, c.slot, win, dx, dy, dz,
-                                                                  margin)))) {
-            return nearest64<DIM>(s, px, py, pz, __longlong_as_double(0x7ff0000000000000LL)).slot;
+    bool per_thread = ties == 0u;
+    int win = -1;
+    if (ties) {
+        const int from = __ffs(static_cast<int>(ties)) - 1;
+        win = __shfl_sync(kAll, c.slot, from);
+        if ((ties & (ties - 1u)) || __any_sync(kAll, mine && c.split)) {
+            const double dx = c.x - __shfl_sync(kAll, c.x, from);
+            const double dy = c.y - __shfl_sync(kAll, c.y, from);
+            const double dz = DIM == 3 ? c.z - __shfl_sync(kAll, c.z, from) : 0.0;
+            per_thread = __any_sync(
+                kAll, mine && (c.split || tie_matters<DIM>(s, c.slot, win, dx, dy, dz, margin)));
+            win = static_cast<int>(
+                __reduce_min_sync(kAll, mine ? static_cast<unsigned>(c.slot) : 0xffffffffu));
         }
-        win = static_cast<int>(
-            __reduce_min_sync(kAll, mine ? static_cast<unsigned>(c.slot) : 0xffffffffu));
+    }
+    if (per_thread) {
+        win = nearest64<DIM>(s, px, py, pz, __longlong_as_double(0x7ff0000000000000LL)).slot;
     }
     return win;
 }
@@ -201,9 +220,10 @@ __device__ __forceinline__ int warp_nearest64_full(const SceneView &s, const Wid
     constexpr unsigned kAll = 0xffffffffu;
     const int lane = static_cast<int>(threadIdx.x & 31u);
     LaneNearest c{__longlong_as_double(0x7ff0000000000000LL), 0.0, 0.0, 0.0, -1, false};
-    float limit = INFINITY, ubest = INFINITY;
-    visit_clusters<DIM>(w, static_cast<float>(px), static_cast<float>(py),
-                        static_cast<float>(pz), limit, [&](int cluster) {
+    const float fx = static_cast<float>(px), fy = static_cast<float>(py);
+    const float fz = static_cast<float>(pz);
+    float limit = first_limit(fx, fy, fz), ubest = INFINITY;
+    visit_clusters<DIM>(w, fx, fy, fz, limit, [&](int cluster) {
         const int ws = cluster * 32 + lane;
         double d2 = __longlong_as_double(0x7ff0000000000000LL);
         if (ws < w.n) {
@@ -292,7 +312,7 @@ __device__ __forceinline__ Candidates warp_candidates64(const SceneView &s, cons
     const float reach = DIM == 2 ? 0.5f * margin : margin;
     float first = INFINITY, second = INFINITY;  // this lane's two smallest bounds
     int ws = 0;
-    float limit = INFINITY, ubest = INFINITY;
+    float limit = first_limit(fx, fy, fz), ubest = INFINITY;
     visit_clusters<DIM>(w, fx, fy, fz, limit, [&](int cluster) {
         float lower;
         const float d = lane_distance<DIM>(w, cluster, fx, fy, fz, lower);
