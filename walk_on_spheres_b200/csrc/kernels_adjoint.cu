@@ -235,9 +235,9 @@ struct HeatPool {
     __device__ __forceinline__ int &slot(int i) {
         return reinterpret_cast<int *>(words())[2 * kHeatPool + i];
     }
-    __device__ __forceinline__ float &radius(int i) {
-        return reinterpret_cast<float *>(words())[2 * kHeatPool + i];
-    }
+    // a walk to be resumed has its radius in the slot's place
+    __device__ __forceinline__ void put_radius(int i, float r) { slot(i) = __float_as_int(r); }
+    __device__ __forceinline__ float radius(int i) { return __int_as_float(slot(i)); }
     __device__ __forceinline__ float &x(int k, int i) {
         return reinterpret_cast<float *>(words())[(3 + k) * kHeatPool + i];
     }
@@ -556,6 +556,8 @@ __device__ __forceinline__ void heat_task32(const HeatArgs &a, const WideView &w
             go_on = !stop;
             ended = stop;
         }
+        // the walks that go on are written to slots that other lanes read above
+        __syncwarp();
         if (adj) {
             // the ended walks' derivatives, summed over the warp
 #pragma unroll
@@ -578,7 +580,7 @@ __device__ __forceinline__ void heat_task32(const HeatArgs &a, const WideView &w
                 const int k2 = kHeatPool - 1 - resume - __popc(back & lt_mask);
                 pool.steps(k2) = qsteps;
                 pool.walk(k2) = qwalk;
-                pool.radius(k2) = qR;
+                pool.put_radius(k2, qR);
                 pool.x(0, k2) = q.x;
                 pool.x(1, k2) = q.y;
                 if (DIM == 3) pool.x(2, k2) = q.z;
