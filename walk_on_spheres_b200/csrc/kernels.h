@@ -66,8 +66,9 @@ struct FastPlan {
     int threads;          // block size
     bool stage_scene;     // copy the wide FP32 boxes into shared memory
     bool stage_prims;     // ... and the wide FP32 primitives
-    int smem_bytes;
+    int smem_bytes;       // of the staged scene: at most kMaxStagedBytes
 };
+constexpr int kMaxStagedBytes = 96 * 1024;
 
 // Per-task partial statistics written by the fast kernel.
 struct TaskPartial {

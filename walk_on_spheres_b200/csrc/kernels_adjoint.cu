@@ -881,8 +881,10 @@ cudaError_t launch_heat_dim(const HeatArgs &a, int precision, const FastPlan &pl
             // the warps' pools (24 KB, adjoint pass 46 KB) and the staged scene
             const int smem =
                 plan.smem_bytes + 8 * 8 * HeatPool::doubles(a.adjoint != 0);
+            // (the largest of both passes and all plans, as in kernels_fast.cu)
             cudaError_t e = cudaFuncSetAttribute(
-                k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+                k, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                kMaxStagedBytes + 8 * 8 * HeatPool::doubles(true));
             if (e != cudaSuccess) return e;
             e = grid_for(k, smem, blocks);
             if (e != cudaSuccess) return e;

@@ -900,10 +900,12 @@ cudaError_t launch_fast_typed(const FastArgs &a, const EqDesc &e, int precision,
             constexpr int HC = decltype(h)::value;
             constexpr int kMinBlocks = min_blocks32<Eq, HC>();
             auto k = walk_fast_kernel<DIM, Eq, float, kMinBlocks, HC>;
-            // (the walk pools are static shared memory beside it)
+            // (the walk pools are static shared memory beside it).  The
+            // limit is the kernel's, not the launch's: always the largest a
+            // plan asks for, so that no thread lowers it under another's launch
             if (plan.smem_bytes > 0) {
                 cudaError_t err = cudaFuncSetAttribute(
-                    k, cudaFuncAttributeMaxDynamicSharedMemorySize, plan.smem_bytes);
+                    k, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxStagedBytes);
                 if (err != cudaSuccess) return err;
             }
             cudaError_t err = grid_for(k, plan.smem_bytes, blocks);
@@ -1721,7 +1723,7 @@ FastPlan plan_fast(const SceneView &s, const WideView &w, long long n_points, in
     // and 0.99; blob of 60k triangles, boxes alone 84 KB: 4.29 and 3.30).
     const size_t box_bytes = 4 * static_cast<size_t>(w.box_total);
     const size_t prim_bytes = 4 * static_cast<size_t>(w.dim == 2 ? 5 : 16) * w.npad;
-    const size_t cap = std::min<size_t>(96 * 1024, smem_optin);
+    const size_t cap = std::min<size_t>(kMaxStagedBytes, smem_optin);
     const bool lists = w.gl != nullptr;
     p.stage_scene = precision == 32 &&
                     (lists ? box_bytes + prim_bytes <= 24 * 1024 : box_bytes <= cap);
