@@ -68,7 +68,7 @@ struct FastPlan {
     bool stage_prims;     // ... and the wide FP32 primitives
     int smem_bytes;       // of the staged scene: at most kMaxStagedBytes
 };
-constexpr int kMaxStagedBytes = 96 * 1024;
+constexpr int kMaxStagedBytes = 24 * 1024;
 
 // Per-task partial statistics written by the fast kernel.
 struct TaskPartial {

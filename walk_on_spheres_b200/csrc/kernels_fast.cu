@@ -1717,10 +1717,12 @@ FastPlan plan_fast(const SceneView &s, const WideView &w, long long n_points, in
     p.chunks = (n_walks + p.chunk - 1) / p.chunk;
     p.n_tasks = n_points * p.chunks;
     // Stage the wide boxes, and the primitives too when they fit, in shared
-    // memory.  With near-boundary lists the tree is hardly read, so only a
-    // scene that costs no resident block is staged, and whole (disk of 1024
-    // segments, 21.5 KB: 7.10 ms staged, 7.25 not; star of 3000, 71 KB: 1.40
-    // and 0.99; blob of 60k triangles, boxes alone 84 KB: 4.29 and 3.30).
+    // memory, where that costs no resident block beside the walk pools (20 to
+    // 27 KB a block).  ms staged / not: with near-boundary lists, which leave
+    // the tree hardly read, a disk of 1024 segments, 21.5 KB, 7.10 / 7.25, star
+    // of 3000, 71 KB, 1.40 / 0.99; without lists a circle of 300 segments, 7
+    // KB, 2.23 / 2.29, of 1000, 21 KB, 2.25 / 2.39, of 3000, its boxes alone
+    // 2.95 / 3.01, whole 3.65; slab of 1384 triangles, 90 KB, 47.4 / 21.5.
     const size_t box_bytes = 4 * static_cast<size_t>(w.box_total);
     const size_t prim_bytes = 4 * static_cast<size_t>(w.dim == 2 ? 5 : 16) * w.npad;
     const size_t cap = std::min<size_t>(kMaxStagedBytes, smem_optin);
