@@ -66,7 +66,6 @@ cudaError_t DeviceBuffer::reserve(size_t n) {
 wos_context::~wos_context() {
     for (DeviceBuffer *b : all_buffers()) b->release();
     sdev.release();
-    if (staging) cudaFreeHost(staging);
     for (auto &ev : events) {
         if (ev) cudaEventDestroy(ev);
     }
@@ -501,21 +500,13 @@ int wos_context::finish_solve(DeviceCounters &hc, const HostFields *host, bool &
         WOS_CUDA(this, cudaStreamSynchronize(stream), "solve");
         return WOS_OK;
     }
-    if (bytes > staging_bytes) {
-        // grown in steps of 64 KB up to kStaging, kept for the context's solves
-        const size_t want = (bytes + 65535) / 65536 * 65536;
-        if (staging) cudaFreeHost(staging);
-        staging = nullptr;
-        staging_bytes = 0;
-        WOS_CUDA(this, cudaMallocHost(&staging, want), "staging block");
-        staging_bytes = want;
-    }
-    WOS_CUDA(this, cudaMemcpyAsync(staging, packed.ptr, bytes, cudaMemcpyDeviceToHost, stream),
-             "read results");
+    if (staging.size() < bytes) staging.resize(bytes);
+    WOS_CUDA(this, cudaMemcpyAsync(staging.data(), packed.ptr, bytes, cudaMemcpyDeviceToHost,
+                                   stream), "read results");
     WOS_CUDA(this, cudaStreamSynchronize(stream), "solve");
-    std::memcpy(&hc, staging, sizeof(hc));
+    std::memcpy(&hc, staging.data(), sizeof(hc));
     if (hc.error_flags) return WOS_OK;  // the caller reports; nothing is handed out
-    const char *at = static_cast<const char *>(staging) + kHeader;
+    const char *at = staging.data() + kHeader;
     for (double *to : {host->mean, host->variance, host->se, host->steps}) {
         if (to) std::memcpy(to, at, sizeof(double) * n);
         at += sizeof(double) * n;

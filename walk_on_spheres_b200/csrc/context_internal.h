@@ -132,10 +132,13 @@ struct wos_context {
     // fields end to end, so a small result comes back in one copy
     static constexpr size_t kHeader = 256;
     wosb::DeviceBuffer packed;
-    // page-locked landing place of such a copy: at most kStaging bytes
-    static constexpr size_t kStaging = size_t(1) << 20;
-    void *staging = nullptr;
-    size_t staging_bytes = 0;
+    // landing place of such a copy: at most kStaging bytes.  Pageable: a
+    // page-locked block saves a repeated call 2 us at 48 points and 31 at 8000,
+    // but its allocation costs a context's first call 2 ms, and 2.5 ms each time
+    // it grows.  us a call of 1 / 8000 / 16 000 / 31 000 points in one copy 78 /
+    // 177 / 280 / 450, in five 146 / 236 / 295 / 421: hence the limit.
+    static constexpr size_t kStaging = size_t(1) << 19;
+    std::vector<char> staging;
     // kernel-level checks
     wosb::DeviceBuffer scratch_a, scratch_b, scratch_c, scratch_d;
     // Gaussian heat source: vertex values, probe weights, gradients, Jacobian
