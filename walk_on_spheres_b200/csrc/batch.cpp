@@ -441,24 +441,29 @@ cudaError_t wos_batch::enqueue() {
         return families[a].n_tasks > families[b].n_tasks;
     });
     const size_t forks = families.size() > 1 ? families.size() - 1 : 0;
-    if (forks > 0) {
-        if ((e = cudaEventRecord(joins.back(), s)) != cudaSuccess) return e;
-        for (size_t k = 0; k < forks; ++k) {
-            if ((e = cudaStreamWaitEvent(side[k], joins.back(), 0)) != cudaSuccess) return e;
-        }
+    cudaError_t failed = cudaSuccess;  // the first error
+    auto done = [&failed](cudaError_t r) {
+        if (failed == cudaSuccess) failed = r;
+        return r == cudaSuccess;
+    };
+    size_t forked = 0;
+    if (forks > 0 && done(cudaEventRecord(joins.back(), s))) {
+        while (forked < forks && done(cudaStreamWaitEvent(side[forked], joins.back(), 0))) ++forked;
     }
-    cudaError_t failed = cudaSuccess;
-    for (size_t k = 0; k < by_size.size(); ++k) {
+    for (size_t k = 0; k < by_size.size() && failed == cudaSuccess; ++k) {
         const size_t f = by_size[k];
         const Family &fam = families[f];
-        e = launch_walk_batch(fam.dim, fam.kind, fam.precision, fam.hc, di + fam.first, fam.count,
-                              fam.n_tasks, q + f, fam.blocks, k == 0 ? s : side[k - 1]);
-        if (e != cudaSuccess) failed = e;
+        done(launch_walk_batch(fam.dim, fam.kind, fam.precision, fam.hc, di + fam.first, fam.count,
+                               fam.n_tasks, q + f, fam.blocks, k == 0 ? s : side[k - 1]));
     }
-    // every fork is joined, also after a failed launch
-    for (size_t k = 0; k < forks; ++k) {
-        if ((e = cudaEventRecord(joins[k], side[k])) != cudaSuccess) return e;
-        if ((e = cudaStreamWaitEvent(s, joins[k], 0)) != cudaSuccess) return e;
+    // every forked stream is joined, after an error too: the caller may release
+    // or replan the buffers once its own stream is idle.  One that cannot be
+    // joined is waited for.
+    for (size_t k = 0; k < forked; ++k) {
+        if (!done(cudaEventRecord(joins[k], side[k])) ||
+            !done(cudaStreamWaitEvent(s, joins[k], 0))) {
+            cudaStreamSynchronize(side[k]);
+        }
     }
     if (failed != cudaSuccess) return failed;
     return launch_merge_batch(di, n, n_points, s);
