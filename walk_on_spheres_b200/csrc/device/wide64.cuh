@@ -419,6 +419,24 @@ __device__ __forceinline__ bool ray_reaches(const SceneView &s, const double *p,
     return true;
 }
 
+// 1 / the ray's component, which is finite also where the component is zero or
+// vanishes in FP32: with an infinite reciprocal a box whose padded face holds
+// the origin would be lost to 0 * inf.
+__host__ __device__ __forceinline__ float ray_reciprocal(double ray) {
+    const float r = static_cast<float>(ray);
+    return 1.0f / (fabsf(r) < 1e-30f ? copysignf(1e-30f, r) : r);
+}
+
+// Narrows the ray's interval [t0, t1] to the slab between lo and hi (relative
+// to the origin).  Along the slab an origin in it keeps the interval, and one
+// off it leaves t0 > t1 for every t that the other slabs allow.
+__host__ __device__ __forceinline__ void clip_to_slab(float lo, float hi, float inv, float &t0,
+                                                      float &t1) {
+    const float ta = lo * inv, tb = hi * inv;
+    t0 = fmaxf(t0, fminf(ta, tb));
+    t1 = fminf(t1, fmaxf(ta, tb));
+}
+
 // count_ray_hits by the whole warp: FP32 tests of the wide tree's boxes,
 // padded by `pad` for their rounding, choose the leaf clusters, and the lanes
 // test a cluster's triangles in FP64.  A triangle that is crossed plainly is
@@ -433,19 +451,14 @@ __device__ __forceinline__ int warp_ray_hits(const SceneView &s, const WideView 
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
         o[k] = static_cast<float>(p[k]);
-        inv[k] = 1.0f / static_cast<float>(ray[k]);
+        inv[k] = ray_reciprocal(ray[k]);
     }
     auto meets = [&](int h, int parent) -> bool {
         const float *b = w.box + w.off[h] + parent * (11 * 32) + lane;
         float t0 = 0.0f, t1 = INFINITY;
 #pragma unroll
         for (int k = 0; k < 3; ++k) {
-            const float lo = b[32 * k] - pad - o[k], hi = b[32 * (3 + k)] + pad - o[k];
-            // a ray along the slab (1 / 0): fminf and fmaxf pass over the NaN
-            // of 0 * inf, and an origin off the slab gives an empty interval
-            const float ta = lo * inv[k], tb = hi * inv[k];
-            t0 = fmaxf(t0, fminf(ta, tb));
-            t1 = fminf(t1, fmaxf(ta, tb));
+            clip_to_slab(b[32 * k] - pad - o[k], b[32 * (3 + k)] + pad - o[k], inv[k], t0, t1);
         }
         // (padding children have lo = inf, hi = -inf)
         return t0 <= t1 * (1.0f + 0x1p-20f) && b[0] < INFINITY;
