@@ -15,6 +15,7 @@ import numpy as np
 import pytest
 
 from walk_on_spheres_b200 import meshes
+from walk_on_spheres_b200._lib import Grid, WosError
 from walk_on_spheres_b200.heat import HeatProblem
 from walk_on_spheres_b200.meshes import Mesh
 
@@ -96,3 +97,55 @@ def test_walks_that_leave_an_open_surface(solver, oracle):
         assert np.array_equal(r.location, ref.location.reshape(r.location.shape))
         assert np.isfinite(r.mean[r.location == 1]).all()
         assert abs(r.counters["max_steps_hits"] - hits) <= 5.0 * np.sqrt(2.0 * n * q * (1.0 - q))
+
+
+@pytest.mark.parametrize("dim", [2, 3])
+def test_grids_whose_spacing_overflows(solver, dim):
+    """Their first coordinates are NaN, the others infinite.  In 2D all are
+    outside; a 3D ray from such a point may cross anything, but the call returns
+    (walks from there find no primitive, which is an error) and the context
+    stays usable."""
+    m = MESHES["height3_2d" if dim == 2 else "height4_3d"]()
+    solver.set_mesh(m)
+    near, _ = _points(dim)
+    want = solver.solve_points("laplace", near, N_walks=16, seed=3, method="fast")
+    for lim in (1e19, 1e21, 1e300, 1.7e308):
+        for yz in (lim, 0.5):
+            grid = Grid(3, 3, 3 if dim == 3 else 1, -lim, lim, -yz, yz, -yz, yz)
+            expected = np.zeros((3, 3, 3 if dim == 3 else 1), dtype=np.uint8)
+            if lim < 1.7e308:  # the middle of each axis is 0
+                if yz == 0.5:
+                    expected[1] = 1
+                else:
+                    expected[(1,) * dim] = 1
+            for method in ("fast", "fast64", "plain"):
+                kw = dict(N_walks=2, seed=1, method=method, max_steps=50)
+                try:
+                    r = solver.solve_grid("laplace", grid=grid, **kw)
+                except WosError:
+                    assert dim == 3 and lim == 1.7e308
+                    continue
+                if dim == 2 or lim < 1.7e308:
+                    assert np.array_equal(r.location, expected)
+    again = solver.solve_points("laplace", near, N_walks=16, seed=3, method="fast")
+    assert np.array_equal(again.mean, want.mean)
+
+
+def test_fp32_walks_that_leave_an_open_surface(solver, oracle):
+    """Counts at a step cap that they reach within FP32's range, as above; with
+    a higher cap their distances overflow, which is an error."""
+    from oracle.oracle import Solve
+    m = _open_sphere()
+    solver.set_mesh(m)
+    kw = dict(N_walks=12, seed=7, max_steps=60)
+    ref = oracle.solve_grid("laplace", Solve(m, 7, 7, 7, **kw))
+    n = 12 * int((ref.location == 1).sum())
+    hits = ref.counters["max_steps_hits"]
+    q = hits / n
+    assert 0.05 < q < 0.95
+    r = solver.solve_grid("laplace", 7, 7, 7, method="fast", **kw)
+    assert abs(r.counters["max_steps_hits"] - hits) <= 5.0 * np.sqrt(2.0 * n * q * (1.0 - q))
+    with pytest.raises(WosError):
+        solver.solve_grid("laplace", 7, 7, 7, method="fast", N_walks=12, seed=7, max_steps=900)
+    again = solver.solve_grid("laplace", 7, 7, 7, method="fast", **kw)
+    assert np.array_equal(again.mean, r.mean, equal_nan=True)

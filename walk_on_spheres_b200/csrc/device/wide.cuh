@@ -417,12 +417,17 @@ inline auto with_height_class(int hc, F &&f) {
 
 // Closest primitive to (px, py, pz); all 32 lanes of the warp must call this
 // with the same point and receive the same result.  HC: the height class the
-// caller guarantees (height_class(w.H) == HC), or kHeightAny.
+// caller guarantees (height_class(w.H) == HC), or kHeightAny.  Slot -1: no
+// finite distance (a point too far away to square, or NaN).
 template <int DIM, int HC = kHeightAny>
 __device__ __forceinline__ WideResult wide_nearest(const WideView &w, float px, float py,
                                                    float pz, float keep, float exact2) {
     constexpr unsigned kAll = 0xffffffffu;
     const unsigned lane = threadIdx.x & 31u;
+    // wide_box_dist puts a NaN point at distance 0 from every child (fmaxf passes
+    // over it), padding children included, which have no nodes of their own
+    const float sum = px + py + pz;
+    if (sum != sum) return WideResult{INFINITY, -1};
     float best = INFINITY, limit = INFINITY;
     int slot = -1;
     auto leaf = [&](int cluster) {

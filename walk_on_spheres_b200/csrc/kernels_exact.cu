@@ -230,8 +230,10 @@ __device__ __forceinline__ int warp_classify_3d(const SceneView &s, const WideVi
                                                 int &retries) {
     const float far = static_cast<float>(fmax(fabs(p[0]), fmax(fabs(p[1]), fabs(p[2]))));
     const float pad = fmaxf(w.margin64, 4e-6f * far);
+    const bool reach = fp32_reaches(static_cast<float>(p[0]), static_cast<float>(p[1]),
+                                    static_cast<float>(p[2]));
     auto count = [&](const double *ray, bool &amb) {
-        return far < 1e9f ? warp_ray_hits(s, w, p, ray, pad, amb) : count_ray_hits(s, p, ray, amb);
+        return reach ? warp_ray_hits(s, w, p, ray, pad, amb) : count_ray_hits(s, p, ray, amb);
     };
     return classify_3d(bdist, btol, max_ray_attempts, rng, retries, count);
 }
