@@ -149,3 +149,26 @@ def test_fp32_walks_that_leave_an_open_surface(solver, oracle):
         solver.solve_grid("laplace", 7, 7, 7, method="fast", N_walks=12, seed=7, max_steps=900)
     again = solver.solve_grid("laplace", 7, 7, 7, method="fast", **kw)
     assert np.array_equal(again.mean, r.mean, equal_nan=True)
+
+
+@pytest.mark.parametrize("name", MESHES)
+def test_closest_points_of_far_points(solver, name):
+    """FP64 distances up to the largest whose square is finite, FP32 ones to a
+    relative 1e-5 (the coordinates' and squares' rounding) up to FP32's range;
+    beyond it, and for NaN, no primitive: infinity and boundary id -1."""
+    m = MESHES[name]()
+    solver.set_mesh(m)
+    x = np.array([1e3, 1e10, 1e18, 3e19, 1e30, 1e150, 1e160, np.nan])
+    pts = np.zeros((len(x), m.dim))
+    pts[:, 0] = x
+    pts[-1] = np.nan
+    reach = np.max(m.verts[:, 0])
+    for precision, last in ((64, 5), (32, 2)):
+        dist, near, bid = solver.closest_points(pts, precision=precision)
+        want = np.where(np.arange(len(x)) <= last, x - reach, np.inf)
+        ok = np.isfinite(want)
+        assert np.all(np.abs(dist[ok] - want[ok]) <= 1e-5 * want[ok])
+        assert np.array_equal(np.isinf(dist), ~ok)
+        assert np.all(near[~ok] == 0.0)
+        if bid is not None:
+            assert np.all(bid[~ok] == -1)

@@ -839,10 +839,11 @@ __global__ void closest32_kernel(SceneView s, WideView w, const double *pts, lon
         }
     }
     if (!valid) return;
-    dist[t] = sqrtf(mybest);
-    V3<double> np;
+    // no primitive at a finite distance (myslot -1): as the FP64 query answers
+    dist[t] = myslot >= 0 ? sqrtf(mybest) : INFINITY;
+    V3<double> np{0.0, 0.0, 0.0};
     int b = -1;
-    reproject64<DIM>(s, w.wide2bin[myslot], px, py, pz, np, b);
+    if (myslot >= 0) reproject64<DIM>(s, w.wide2bin[myslot], px, py, pz, np, b);
     nearest[DIM * t] = np.x;
     nearest[DIM * t + 1] = np.y;
     if (DIM == 3) nearest[DIM * t + 2] = np.z;
