@@ -172,3 +172,25 @@ def test_closest_points_of_far_points(solver, name):
         assert np.all(near[~ok] == 0.0)
         if bid is not None:
             assert np.all(bid[~ok] == -1)
+
+
+@pytest.mark.parametrize("name", ["height2_2d", "height3_2d", "height3_3d", "height4_3d"])
+def test_scenes_whose_fp32_distances_overflow(solver, name):
+    """A mesh 2^66 times as large: its lattice and lists hold no finite distance,
+    so FAST_FP32 walks find no primitive (an error) and read nothing.  FP64
+    walks are those of the unit mesh, scaled: equal steps, and g = x^2 - y^2 (2D)
+    and a degree-5 harmonic (3D) scale exactly."""
+    m = MESHES[name]()
+    f = 2.0 ** 66
+    near, _ = _points(m.dim)
+    kw = dict(N_walks=8, seed=3, max_steps=100)
+    solver.set_mesh(m)
+    want = solver.solve_points("laplace", near, method="plain", epsilon=1e-2, **kw)
+    solver.set_mesh(Mesh(m.dim, m.verts * f, m.prims, m.boundary_ids))
+    with pytest.raises(WosError):
+        solver.solve_points("laplace", near * f, method="fast", epsilon=1e-2 * f, **kw)
+    r = solver.solve_points("laplace", near * f, method="plain", epsilon=1e-2 * f, **kw)
+    assert np.array_equal(r.location, want.location)
+    assert np.array_equal(r.mean_steps, want.mean_steps)
+    g = f ** 2 if m.dim == 2 else f ** 5
+    assert np.all(np.abs(r.mean / g - want.mean) <= 1e-9 * np.maximum(1.0, np.abs(want.mean)))

@@ -30,6 +30,7 @@
 // radius whose ball lies inside the domain.  Below exact2 (inside the
 // epsilon shell) pruning is exact.
 #pragma once
+#include <cfloat>
 #include <cstdint>
 #include <type_traits>
 
@@ -334,6 +335,8 @@ __device__ __forceinline__ WideResult warp_list_nearest(const WideView &w, bool 
 // ascending order go to out[0 .. cap) and their count to every lane.  Once
 // more than cap are found the search stops and returns a count above cap.
 // Children are visited when their lower bound (box and slab) is within r2.
+// Only finite distances count: a scene whose FP32 squares overflow asks with an
+// infinite r2, and padding children (no nodes of their own) lie at infinity.
 template <int DIM>
 __device__ int wide_range(const WideView &w, float px, float py, float pz, float r2, int *out,
                           int cap) {
@@ -341,6 +344,7 @@ __device__ int wide_range(const WideView &w, float px, float py, float pz, float
     const unsigned lane = threadIdx.x & 31u;
     const unsigned below = (1u << lane) - 1u;
     int count = 0;
+    r2 = fminf(r2, FLT_MAX);
     auto leaf = [&](int cluster) {
         const float d2 = wide_prim_dist<DIM>(w, cluster, px, py, pz);
         const unsigned m = __ballot_sync(kAll, d2 <= r2);
