@@ -181,8 +181,8 @@ __device__ __forceinline__ float log_k0<float>(float x) {
 
 // The same approximants with the hardware's approximate logarithm, reciprocal
 // and root, for tests that settle a close call with the forms above: K0(x) for
-// 0 < x <= 2, ln I0(x) and ln K0(x) for x > 0, within about 1e-6 of K0 or
-// (1 + x) 1e-6 of the logarithms.
+// 0 < x <= 2, ln I0(x) and ln K0(x) for x > 0.  What they may differ by there is
+// said, with the measurement, at the test (sc_accepts_2d).
 __device__ __forceinline__ float quick_k0_small(float x, float i0) {
     return as_k0_rest(0.25f * x * x) - __logf(0.5f * x) * i0;
 }
