@@ -407,16 +407,23 @@ __host__ __device__ __forceinline__ int traversal_class(const WideView &w) {
     return w.n <= lane_prims(w.dim) ? kLaneScan : height_class(w.H);
 }
 
-// Host dispatch: calls f(std::integral_constant<int, HC>{}) for class hc.
+// Host dispatch: calls f(std::integral_constant<int, HC>{}) for class hc, a
+// height_class; every class is one more kernel to load in a process's first
+// call.
 template <class F>
 inline auto with_height_class(int hc, F &&f) {
     switch (hc) {
-        case kLaneScan: return f(std::integral_constant<int, kLaneScan>{});
         case kHeightUpTo2: return f(std::integral_constant<int, kHeightUpTo2>{});
         case kHeight3: return f(std::integral_constant<int, kHeight3>{});
         case kHeight4: return f(std::integral_constant<int, kHeight4>{});
         default: return f(std::integral_constant<int, kHeightOther>{});
     }
+}
+// The same for a traversal_class.
+template <class F>
+inline auto with_traversal_class(int hc, F &&f) {
+    if (hc == kLaneScan) return f(std::integral_constant<int, kLaneScan>{});
+    return with_height_class(hc, f);
 }
 
 // Closest primitive to (px, py, pz); all 32 lanes of the warp must call this

@@ -744,7 +744,7 @@ cudaError_t batch_typed(int precision, int hc, const BatchItem *items, int n_ite
                         long long n_tasks, unsigned long long *queue, int blocks,
                         cudaStream_t stream) {
     if (precision == 32) {
-        return with_height_class(hc, [&](auto h) {
+        return with_traversal_class(hc, [&](auto h) {
             constexpr int HC = decltype(h)::value;
             constexpr int kMinBlocks = min_blocks32<Eq, HC>();
             walk_batch_kernel<DIM, Eq, float, kMinBlocks, HC><<<blocks, 256, 0, stream>>>(
@@ -762,7 +762,7 @@ cudaError_t batch_blocks_typed(int precision, int hc, int &blocks) {
     int per_sm = 0, dev = 0, sms = 0;
     cudaError_t e;
     if (precision == 32) {
-        e = with_height_class(hc, [&](auto h) {
+        e = with_traversal_class(hc, [&](auto h) {
             constexpr int HC = decltype(h)::value;
             constexpr int kMinBlocks = min_blocks32<Eq, HC>();
             return cudaOccupancyMaxActiveBlocksPerMultiprocessor(
@@ -897,7 +897,7 @@ cudaError_t launch_fast_typed(const FastArgs &a, const EqDesc &e, int precision,
     };
     int blocks = 0;
     if (precision == 32) {
-        return with_height_class(traversal_class(a.w), [&](auto h) -> cudaError_t {
+        return with_traversal_class(traversal_class(a.w), [&](auto h) -> cudaError_t {
             constexpr int HC = decltype(h)::value;
             constexpr int kMinBlocks = min_blocks32<Eq, HC>();
             auto k = walk_fast_kernel<DIM, Eq, float, kMinBlocks, HC>;
