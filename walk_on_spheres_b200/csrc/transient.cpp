@@ -279,10 +279,12 @@ extern "C" int wos_transient_solve(wos_context *ctx, const wos_transient_params 
     if (p.method != WOS_METHOD_PLAIN_FP64) {
         plan = plan_fast(dev.view, dev.wide, n, p.walks, precision, ctx->sms, ctx->smem_optin);
         // a step is small: about two waves of tasks, and at least 256 walks
-        // (8 per lane) per task so that a lane whose walk ends takes the
-        // next one.  At the level-2 defaults 32 walks per task (one per
-        // lane) left a warp waiting for its longest walk: 276 ms for the
-        // run, against 184 ms at 256.
+        // (8 per lane) per task so that a lane whose walk waits takes the
+        // next one.  25 steps at 64 / 128 / 256 / 512 walks per task, ms: 49 x
+        // 33 points x 500 walks 34.8 / 28.1 / 25.8 / 40.4, 97 x 65 x 500 125 /
+        // 114 / 77 / 74, 97 x 65 x 2000 481 / 347 / 283 / 253 (1024: 242).  Only
+        // on plates that leave most warps idle are shorter tasks better (25 x 17
+        // x 500 13.5 / 15.9 / 22.9 / 36.7).
         const long long resident = static_cast<long long>(ctx->sms) * 24;
         long long chunk = static_cast<long long>(p.walks) * n / (2 * resident);
         chunk = std::max<long long>(256, std::min<long long>(1024, chunk));
