@@ -302,6 +302,30 @@ __device__ __forceinline__ void write_heat_partial(const HeatArgs &a, unsigned l
     }
 }
 
+// list_nearest of a 2D list, its roundings spelled out.  Left to the compiler,
+// which product of the dot product is fused depends on the code around it, and
+// a radius that differs in the last bit moves a walk.
+__device__ __forceinline__ WideResult segment_list_nearest(const WideView &w, const int *list,
+                                                           int k, float px, float py) {
+    float best = INFINITY;
+    int slot = -1;
+    for (int q = 0; q < k; ++q) {
+        const int s = __ldg(list + q);
+        const float4 a = __ldg(w.aos + 2 * s);
+        const float inv = __ldg(reinterpret_cast<const float *>(w.aos + 2 * s + 1));
+        const float wx = px - a.x, wy = py - a.y;
+        const float dot = __fmaf_rn(wy, a.w, __fmul_rn(wx, a.z));
+        const float t = fminf(fmaxf(__fmul_rn(dot, inv), 0.0f), 1.0f);
+        const float dx = __fmaf_rn(-t, a.z, wx), dy = __fmaf_rn(-t, a.w, wy);
+        const float d2 = __fmaf_rn(dx, dx, __fmul_rn(dy, dy));
+        if (d2 < best) {
+            best = d2;
+            slot = s;
+        }
+    }
+    return WideResult{best, slot};
+}
+
 // One FAST_FP32 task.  Half of these walks' steps query (epsilon is small),
 // so the lists and cooperative queries run in every iteration, for about half
 // of the lanes; but the FP64 re-projection of a step that came within the FP32
@@ -445,8 +469,8 @@ __device__ __forceinline__ void heat_task32(const HeatArgs &a, const WideView &w
         float qbest = 0.0f;
         if constexpr (DIM == 2) {
             if (listed) {
-                const WideResult q = list_nearest<DIM>(wv, list_of(wv, packed),
-                                                       list_length(packed), p.x, p.y, 0.0f);
+                const WideResult q = segment_list_nearest(wv, list_of(wv, packed),
+                                                          list_length(packed), p.x, p.y);
                 qbest = q.best;
                 slot = q.slot;
             }
