@@ -136,7 +136,8 @@ struct wos_context {
     // page-locked block saves a repeated call 2 us at 48 points and 31 at 8000,
     // but its allocation costs a context's first call 2 ms, and 2.5 ms each time
     // it grows.  us a call of 1 / 8000 / 16 000 / 31 000 points in one copy 78 /
-    // 177 / 280 / 450, in five 146 / 236 / 295 / 421: hence the limit.
+    // 177 / 280 / 450, in five 146 / 236 / 295 / 421: hence the limit (arrays that
+    // do not lie end to end).
     static constexpr size_t kStaging = size_t(1) << 19;
     std::vector<char> staging;
     // kernel-level checks
@@ -163,6 +164,15 @@ struct wos_context {
         long long n;
         double *mean, *variance, *se, *steps;
         uint8_t *loc;
+        // whether they lie end to end, as the fields do on the device: one copy
+        // fills them, which pays from 2048 points on (us a call of 1900 / 4000 /
+        // 8000 / 16 000 points through the staging block 107 / 134 / 177 / 280,
+        // straight 112 / 130 / 167 / 240; of 31 000 / 60 000 in five copies 421 /
+        // 650, straight 360 / 590)
+        bool end_to_end() const {
+            return n >= 2048 && mean && variance == mean + n && se == variance + n && steps == se + n &&
+                   loc == reinterpret_cast<uint8_t *>(steps + n);
+        }
     };
     int run(const wos_params &p, const wosb::PointSet &ps, wosb::Fields out, wos_counters *c,
             const HostFields *host = nullptr);
