@@ -8,6 +8,7 @@
 #include <cstdio>
 #include <cstring>
 #include <cstdlib>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -20,7 +21,58 @@ using namespace wosb;
 
 namespace {
 thread_local std::string g_error;
+
+// The Landing block.  Never destroyed: contexts may outlive static objects.
+struct LandingBlock {
+    std::mutex in_use;  // held from take() to give()
+    std::mutex count;
+    int contexts = 0;
+    void *ptr = nullptr;
+    double spent = 0.0;  // us that copies without it have taken longer
+};
+constexpr double kLandingCost = 2000.0;  // us of its allocation
+LandingBlock &landing_block() {
+    static LandingBlock *b = new LandingBlock;
+    return *b;
+}
 }  // namespace
+
+void *Landing::take(size_t bytes) {
+    LandingBlock &b = landing_block();
+    if (!b.in_use.try_lock()) return nullptr;
+    if (!b.ptr) {
+        b.spent += 2.0 + 1.1e-4 * static_cast<double>(bytes);
+        if (b.spent >= kLandingCost) {
+            b.spent = 0.0;  // (also where it cannot be had: ordinary memory serves)
+            if (cudaHostAlloc(&b.ptr, kBytes, cudaHostAllocPortable) != cudaSuccess) {
+                cudaGetLastError();
+                b.ptr = nullptr;
+            }
+        }
+        if (!b.ptr) {
+            b.in_use.unlock();
+            return nullptr;
+        }
+    }
+    return b.ptr;
+}
+
+void Landing::give() { landing_block().in_use.unlock(); }
+
+LandingUse::LandingUse() {
+    LandingBlock &b = landing_block();
+    const std::lock_guard<std::mutex> lock(b.count);
+    ++b.contexts;
+}
+
+LandingUse::~LandingUse() {
+    LandingBlock &b = landing_block();
+    const std::lock_guard<std::mutex> lock(b.count);
+    if (--b.contexts > 0) return;
+    if (b.ptr) cudaFreeHost(b.ptr);  // no context, no solve
+    b.ptr = nullptr;
+    b.spent = 0.0;
+}
 
 std::string wosb::device_error(unsigned flags) {
     std::string m;
@@ -493,26 +545,31 @@ int wos_context::finish_solve(DeviceCounters &hc, const HostFields *host, bool &
     static_assert(sizeof(DeviceCounters) <= kHeader, "the counters fit their header");
     const size_t n = host ? static_cast<size_t>(host->n) : 0;
     const size_t bytes = kHeader + n * (4 * sizeof(double) + 1);
-    fetched = host != nullptr && bytes <= kStaging && !host->end_to_end();
+    void *block = host && bytes <= Landing::kBytes ? Landing::take(bytes) : nullptr;
+    fetched = block || (host && bytes <= kStaging && !host->end_to_end());
     if (!fetched) {
         WOS_CUDA(this, cudaMemcpyAsync(&hc, packed.ptr, sizeof(hc), cudaMemcpyDeviceToHost,
                                        stream), "read counters");
         WOS_CUDA(this, cudaStreamSynchronize(stream), "solve");
         return WOS_OK;
     }
-    if (staging.size() < bytes) staging.resize(bytes);
-    WOS_CUDA(this, cudaMemcpyAsync(staging.data(), packed.ptr, bytes, cudaMemcpyDeviceToHost,
-                                   stream), "solve");
-    // (a copy to pageable memory returns when it has completed)
-    std::memcpy(&hc, staging.data(), sizeof(hc));
-    if (hc.error_flags) return WOS_OK;  // the caller reports; nothing is handed out
-    const char *at = staging.data() + kHeader;
-    for (double *to : {host->mean, host->variance, host->se, host->steps}) {
-        if (to) std::memcpy(to, at, sizeof(double) * n);
-        at += sizeof(double) * n;
+    if (!block && staging.size() < bytes) staging.resize(bytes);
+    const char *at = block ? static_cast<const char *>(block) : staging.data();
+    cudaError_t e = cudaMemcpyAsync(block ? block : staging.data(), packed.ptr, bytes,
+                                    cudaMemcpyDeviceToHost, stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
+    if (e == cudaSuccess) {
+        std::memcpy(&hc, at, sizeof(hc));
+        at += kHeader;
+        // (after a device error the caller reports; nothing is handed out)
+        for (double *to : {host->mean, host->variance, host->se, host->steps}) {
+            if (to && !hc.error_flags) std::memcpy(to, at, sizeof(double) * n);
+            at += sizeof(double) * n;
+        }
+        if (host->loc && !hc.error_flags) std::memcpy(host->loc, at, n);
     }
-    if (host->loc) std::memcpy(host->loc, at, n);
-    return WOS_OK;
+    if (block) Landing::give();
+    return e == cudaSuccess ? WOS_OK : cuda_fail(this, e, "solve");
 }
 
 int wos_context::run(const wos_params &p, const PointSet &ps, Fields out,

@@ -11,6 +11,30 @@
 
 namespace wosb {
 
+// A process's page-locked block for the copies of small results, one solve at
+// a time.  A block per context cost 2 ms (cudaMallocHost) of each context's
+// first solve and 2.5 ms each time it grew; a copy to ordinary memory costs a
+// repeated solve of 48 / 4000 / 8000 / 16 000 points 79 / 134 / 177 / 280 us
+// against 76 / 117 / 146 / 220.  So it is allocated, at its full size, once
+// copies to ordinary memory have cost as much as it does (700 solves of 48
+// points, 120 of 4000), and freed with the process's last context.
+class Landing {
+  public:
+    static constexpr size_t kBytes = size_t(1) << 20;
+    // The block for the calling thread until give(), or null: it is not worth its
+    // allocation yet, another thread has it, or it cannot be allocated.  For a
+    // copy of `bytes` (at most kBytes).
+    static void *take(size_t bytes);
+    static void give();
+};
+// A context's share in the block's life.
+struct LandingUse {
+    LandingUse();
+    ~LandingUse();
+    LandingUse(const LandingUse &) = delete;
+    LandingUse &operator=(const LandingUse &) = delete;
+};
+
 // Grow-only device allocation.
 struct DeviceBuffer {
     void *ptr = nullptr;
@@ -132,12 +156,10 @@ struct wos_context {
     // fields end to end, so a small result comes back in one copy
     static constexpr size_t kHeader = 256;
     wosb::DeviceBuffer packed;
-    // landing place of such a copy: at most kStaging bytes.  Pageable: a
-    // page-locked block saves a repeated call 2 us at 48 points and 31 at 8000,
-    // but its allocation costs a context's first call 2 ms, and 2.5 ms each time
-    // it grows.  us a call of 1 / 8000 / 16 000 / 31 000 points in one copy 78 /
-    // 177 / 280 / 450, in five 146 / 236 / 295 / 421: hence the limit (arrays that
-    // do not lie end to end).
+    wosb::LandingUse landing;
+    // where such a copy lands when the Landing block is taken: at most kStaging
+    // bytes.  us a call of 1 / 8000 / 16 000 / 31 000 points in one copy 78 / 177 /
+    // 280 / 450, in five (separate arrays) 146 / 236 / 295 / 421: hence the limit.
     static constexpr size_t kStaging = size_t(1) << 19;
     std::vector<char> staging;
     // kernel-level checks
@@ -165,10 +187,10 @@ struct wos_context {
         double *mean, *variance, *se, *steps;
         uint8_t *loc;
         // whether they lie end to end, as the fields do on the device: one copy
-        // fills them, which pays from 2048 points on (us a call of 1900 / 4000 /
-        // 8000 / 16 000 points through the staging block 107 / 134 / 177 / 280,
-        // straight 112 / 130 / 167 / 240; of 31 000 / 60 000 in five copies 421 /
-        // 650, straight 360 / 590)
+        // fills them, which beats ordinary staging memory from 2048 points on (us
+        // a call of 1900 / 4000 / 8000 / 16 000 points 112 / 130 / 167 / 240 against
+        // 107 / 134 / 177 / 280; of 31 000 / 60 000 360 / 590, in five copies 421 /
+        // 650)
         bool end_to_end() const {
             return n >= 2048 && mean && variance == mean + n && se == variance + n && steps == se + n &&
                    loc == reinterpret_cast<uint8_t *>(steps + n);

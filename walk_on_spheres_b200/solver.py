@@ -72,7 +72,7 @@ def _enum(value, table, what):
 
 def _fields(n: int) -> list:
     """The five result fields of n points.  From 2048 points on end to end in one
-    block, which the solve fills with one copy (fewer come through a staged one)."""
+    block, which a solve fills with one copy (small ones come through a staged one)."""
     if n < 2048:
         return [np.empty(n) for _ in range(4)] + [np.empty(n, dtype=np.uint8)]
     block = np.empty(33 * n, dtype=np.uint8)
