@@ -194,3 +194,43 @@ def test_scenes_whose_fp32_distances_overflow(solver, name):
     assert np.array_equal(r.mean_steps, want.mean_steps)
     g = f ** 2 if m.dim == 2 else f ** 5
     assert np.all(np.abs(r.mean / g - want.mean) <= 1e-9 * np.maximum(1.0, np.abs(want.mean)))
+
+
+@pytest.mark.parametrize("power", [133, 533])
+@pytest.mark.parametrize("name", ["height1_2d", "height3_2d", "height4_3d"])
+def test_scenes_beyond_fp32(solver, name, power):
+    """Coordinates that FP32 cannot hold (2^133), or whose FP64 squares overflow
+    too (2^533): no lattice; FAST_FP32 fails as above.  FP64 walks at 2^133 are
+    the unit mesh's, scaled; at 2^533 no distance is finite, and 2D calls only
+    have to return (3D meshes are refused: no triangle has a finite area).  The
+    solver stays usable."""
+    m = MESHES[name]()
+    f = 2.0 ** power
+    near, _ = _points(m.dim)
+    kw = dict(N_walks=8, seed=3, max_steps=100)
+    solver.set_mesh(m)
+    want = solver.solve_points("laplace", near, method="plain", epsilon=1e-2, **kw)
+    scaled = Mesh(m.dim, m.verts * f, m.prims, m.boundary_ids)
+    if m.dim == 3 and power == 533:
+        with pytest.raises(WosError):
+            solver.set_mesh(scaled)
+        return
+    solver.set_mesh(scaled)
+    results = {}
+    for method in ("fast", "fast64", "plain"):
+        try:
+            results[method] = solver.solve_points("laplace", near * f, method=method,
+                                                  epsilon=1e-2 * f, **kw)
+        except WosError:
+            assert method == "fast"
+    if power == 133:
+        assert "fast" not in results
+        r = results["plain"]
+        assert np.array_equal(r.location, want.location)
+        assert np.array_equal(r.mean_steps, want.mean_steps)
+        g = f ** 2 if m.dim == 2 else f ** 5
+        assert np.all(np.abs(r.mean / g - want.mean)
+                      <= 1e-9 * np.maximum(1.0, np.abs(want.mean)))
+    solver.set_mesh(m)
+    again = solver.solve_points("laplace", near, method="plain", epsilon=1e-2, **kw)
+    assert np.array_equal(again.mean, want.mean)

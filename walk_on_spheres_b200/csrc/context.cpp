@@ -355,7 +355,8 @@ cudaError_t SceneDevice::build_lattice(const HostScene &h, cudaStream_t stream) 
         ext = std::max(ext, h.bbox[2 * k + 1] - h.bbox[2 * k]);
         mag = std::max({mag, std::fabs(h.bbox[2 * k]), std::fabs(h.bbox[2 * k + 1])});
     }
-    if (!(ext > 0.0)) return cudaSuccess;
+    // (no lattice where FP32 cannot hold the coordinates either)
+    if (!(ext > 0.0) || !(mag < 1e38)) return cudaSuccess;
     const double step = ext / (G - 1);
     int n[3] = {1, 1, 1};
     for (int k = 0; k < h.dim; ++k) {

@@ -337,6 +337,7 @@ __device__ __forceinline__ WideResult warp_list_nearest(const WideView &w, bool 
 // Children are visited when their lower bound (box and slab) is within r2.
 // Only finite distances count: a scene whose FP32 squares overflow asks with an
 // infinite r2, and padding children (no nodes of their own) lie at infinity.
+// A NaN point has none in reach (wide_nearest says why).
 template <int DIM>
 __device__ int wide_range(const WideView &w, float px, float py, float pz, float r2, int *out,
                           int cap) {
@@ -344,6 +345,8 @@ __device__ int wide_range(const WideView &w, float px, float py, float pz, float
     const unsigned lane = threadIdx.x & 31u;
     const unsigned below = (1u << lane) - 1u;
     int count = 0;
+    const float sum = px + py + pz;
+    if (sum != sum) return 0;
     r2 = fminf(r2, FLT_MAX);
     auto leaf = [&](int cluster) {
         const float d2 = wide_prim_dist<DIM>(w, cluster, px, py, pz);

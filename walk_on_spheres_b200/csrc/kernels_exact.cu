@@ -489,7 +489,7 @@ __global__ void __launch_bounds__(kExactThreads)
                 const Nearest<double> q = nearest64<DIM>(s, k.p.x, k.p.y, k.p.z, dinf());
                 k.R = sqrt(q.best);
                 k.np = V3<double>{q.x, q.y, q.z};
-                if (DIM == 2) k.bid = s.segid[q.slot].x;
+                if (DIM == 2) k.bid = q.slot >= 0 ? s.segid[q.slot].x : -1;
             }
             k.end(eq, eps, start);
         }
