@@ -547,7 +547,7 @@ int wos_context::finish_solve(DeviceCounters &hc, const HostFields *host, bool &
     const size_t n = host ? static_cast<size_t>(host->n) : 0;
     const size_t bytes = kHeader + n * (4 * sizeof(double) + 1);
     void *block = host && bytes <= Landing::kBytes ? Landing::take(bytes) : nullptr;
-    fetched = block || (host && bytes <= kStaging && !host->end_to_end());
+    fetched = block || (host && bytes <= kStaging);
     if (!fetched) {
         WOS_CUDA(this, cudaMemcpyAsync(&hc, packed.ptr, sizeof(hc), cudaMemcpyDeviceToHost,
                                        stream), "read counters");
@@ -708,12 +708,6 @@ int wos_context::fields_for(long long n, Fields &out) {
 
 int wos_context::download(const Fields &dev, const HostFields &h) {
     const size_t b = sizeof(double) * static_cast<size_t>(h.n);
-    if (h.end_to_end()) {
-        WOS_CUDA(this, cudaMemcpyAsync(h.mean, dev.mean, 4 * b + static_cast<size_t>(h.n),
-                                       cudaMemcpyDeviceToHost, stream), "D2H");
-        WOS_CUDA(this, cudaStreamSynchronize(stream), "D2H");
-        return WOS_OK;
-    }
     if (h.mean) WOS_CUDA(this, cudaMemcpyAsync(h.mean, dev.mean, b, cudaMemcpyDeviceToHost, stream), "D2H");
     if (h.variance) WOS_CUDA(this, cudaMemcpyAsync(h.variance, dev.variance, b, cudaMemcpyDeviceToHost, stream), "D2H");
     if (h.se) WOS_CUDA(this, cudaMemcpyAsync(h.se, dev.standard_error, b, cudaMemcpyDeviceToHost, stream), "D2H");

@@ -159,7 +159,7 @@ struct wos_context {
     wosb::LandingUse landing;
     // where such a copy lands when the Landing block is taken: at most kStaging
     // bytes.  us a call of 1 / 8000 / 16 000 / 31 000 points in one copy 78 / 177 /
-    // 280 / 450, in five (separate arrays) 146 / 236 / 295 / 421: hence the limit.
+    // 280 / 450, in five 146 / 236 / 295 / 421: hence the limit.
     static constexpr size_t kStaging = size_t(1) << 19;
     std::vector<char> staging;
     // kernel-level checks
@@ -186,15 +186,6 @@ struct wos_context {
         long long n;
         double *mean, *variance, *se, *steps;
         uint8_t *loc;
-        // whether they lie end to end, as the fields do on the device: one copy
-        // fills them, which beats ordinary staging memory from 2048 points on (us
-        // a call of 1900 / 4000 / 8000 / 16 000 points 112 / 130 / 167 / 240 against
-        // 107 / 134 / 177 / 280; of 31 000 / 60 000 360 / 590, in five copies 421 /
-        // 650)
-        bool end_to_end() const {
-            return n >= 2048 && mean && variance == mean + n && se == variance + n && steps == se + n &&
-                   loc == reinterpret_cast<uint8_t *>(steps + n);
-        }
     };
     int run(const wos_params &p, const wosb::PointSet &ps, wosb::Fields out, wos_counters *c,
             const HostFields *host = nullptr);

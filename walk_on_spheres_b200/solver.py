@@ -70,15 +70,6 @@ def _enum(value, table, what):
     return int(value)
 
 
-def _fields(n: int) -> list:
-    """The five result fields of n points.  From 2048 points on end to end in one
-    block, which a solve fills with one copy (small ones come through a staged one)."""
-    if n < 2048:
-        return [np.empty(n) for _ in range(4)] + [np.empty(n, dtype=np.uint8)]
-    block = np.empty(33 * n, dtype=np.uint8)
-    return [block[8 * n * k:8 * n * (k + 1)].view(np.float64) for k in range(4)] + [block[32 * n:]]
-
-
 class Solver:
     """A libwos_b200 context on one CUDA device."""
 
@@ -168,7 +159,8 @@ class Solver:
         g = grid if grid is not None else self.grid_over_mesh(Nx, Ny, Nz)
         shape = (g.Nx, g.Ny, g.Nz if self.dim == 3 else 1)
         n = int(np.prod(shape))
-        res = GridResult(*_fields(n))
+        res = GridResult(np.empty(n), np.empty(n), np.empty(n), np.empty(n),
+                         np.empty(n, dtype=np.uint8))
         c = _lib.Counters()
         p = self.params(equation, **kw)
         self._check(self._L.wos_solve_grid(self._ctx, C.byref(p), C.byref(g), _ptr(res.mean),
@@ -202,7 +194,8 @@ class Solver:
         pts = np.ascontiguousarray(points, dtype=np.float64).reshape(-1, self.dim)
         n = pts.shape[0]
         idx = None if point_index is None else np.ascontiguousarray(point_index, dtype=np.uint64)
-        res = GridResult(*_fields(n))
+        res = GridResult(np.empty(n), np.empty(n), np.empty(n), np.empty(n),
+                         np.empty(n, dtype=np.uint8))
         c = _lib.Counters()
         p = self.params(equation, **kw)
         self._check(self._L.wos_solve_points(self._ctx, C.byref(p), _ptr(pts), _ptr(idx), n,
