@@ -60,6 +60,7 @@ struct HeatArgs {
     int chunk;
     int chunks;
     long long n_tasks;
+    int stage_box, stage_prim;  // floats of a scene in shared memory (0: not staged)
     int mode;
     double Q, x0, y0, z0, inv_s2, inv_s;
     double beta;                            // MIS: probability of a Green sample
@@ -755,15 +756,24 @@ __device__ __forceinline__ void heat_task64(const HeatArgs &a, const WideView &w
 template <int DIM, typename T, int MIN_BLOCKS, int HC>
 __global__ void __launch_bounds__(256, MIN_BLOCKS) heat_walk_kernel(HeatArgs a) {
     constexpr bool kF32 = std::is_same<T, float>::value;
-    extern __shared__ float4 smem[];  // FP32: the warps' pools
+    extern __shared__ float4 smem[];  // FP32: the warps' pools, then a small scene
     __shared__ int s_off[8];
     if (threadIdx.x < 8) s_off[threadIdx.x] = a.w.off[threadIdx.x];
     WideView wv = a.w;
     wv.off = s_off;
     double *pool = nullptr;
     if constexpr (kF32) {
-        pool = reinterpret_cast<double *>(smem) +
-               (threadIdx.x >> 5) * HeatPool::doubles(a.adjoint != 0);
+        const int words = HeatPool::doubles(a.adjoint != 0);
+        pool = reinterpret_cast<double *>(smem) + (threadIdx.x >> 5) * words;
+        if (a.stage_prim) {
+            float *sm = reinterpret_cast<float *>(reinterpret_cast<double *>(smem) + 8 * words);
+            for (int i = threadIdx.x; i < a.stage_box; i += blockDim.x) sm[i] = a.w.box[i];
+            for (int i = threadIdx.x; i < a.stage_prim; i += blockDim.x) {
+                sm[a.stage_box + i] = a.w.prim[i];
+            }
+            wv.box = sm;
+            wv.prim = sm + a.stage_box;
+        }
     }
     __syncthreads();
     const int lane = threadIdx.x & 31;
@@ -860,6 +870,14 @@ __global__ void heat_merge_kernel(HeatArgs a, HeatOut out) {
     }
 }
 
+// Scenes up to this size are staged beside the pools: those without a lattice,
+// where every step queries the tree (circle of 50 segments, 2048 probes x 2048
+// walks: forward / adjoint 7.2 / 7.6 ms staged, 7.6 / 8.0 not).  Larger ones
+// take L1 and resident blocks from the lists and the lattice: with near-boundary
+// lists 1.03 / 1.55 ms staged and 1.01 / 1.24 not (circle of 1000 segments), without
+// 1.50 / 2.05 and 1.50 / 1.78, 13.4 / 13.7 and 6.6 / 7.3 (slab of 1384 triangles).
+constexpr int kHeatStagedBytes = 3 * 1024 + 256;
+
 template <int DIM>
 cudaError_t launch_heat_dim(const HeatArgs &a, int precision, const FastPlan &plan,
                             cudaStream_t stream) {
@@ -888,13 +906,12 @@ cudaError_t launch_heat_dim(const HeatArgs &a, int precision, const FastPlan &pl
             // resident warps pay in spite of spills (slab of 20k triangles,
             // forward / adjoint pass: 17.4 / 19.5 ms, 19.0 / 20.1 at 3)
             auto k = heat_walk_kernel<DIM, float, 4, HC>;
-            // the warps' pools: 24 KB, adjoint pass 45 KB (below the 48 KB that
-            // need no consent).  The scene is not staged beside them: with
-            // near-boundary lists forward / adjoint take 1.03 / 1.55 ms staged
-            // and 1.01 / 1.24 not (circle of 1000 segments), without 1.50 / 2.05
-            // and 1.50 / 1.78, 13.4 / 13.7 and 6.6 / 7.3 (slab of 1384 triangles)
-            const int smem = 8 * 8 * HeatPool::doubles(a.adjoint != 0);
-            static_assert(8 * 8 * HeatPool::doubles(true) + 32 <= 48 * 1024, "no consent");
+            // the warps' pools: 24 KB, adjoint pass 45 KB, and a scene without a
+            // lattice (below the 48 KB that need no consent)
+            const int smem = 8 * 8 * HeatPool::doubles(a.adjoint != 0) +
+                             4 * (a.stage_box + a.stage_prim);
+            static_assert(8 * 8 * HeatPool::doubles(true) + kHeatStagedBytes + 32 <= 48 * 1024,
+                          "no consent");
             cudaError_t e = grid_for(k, smem, blocks);
             if (e != cudaSuccess) return e;
             k<<<blocks, plan.threads, smem, stream>>>(a);
@@ -936,6 +953,10 @@ cudaError_t launch_heat(const SceneView &s, const WideView &w, const PointSet &p
     a.chunk = plan.chunk;
     a.chunks = plan.chunks;
     a.n_tasks = plan.n_tasks;
+    if (w.gl == nullptr && plan.stage_prims && plan.smem_bytes <= kHeatStagedBytes) {
+        a.stage_box = w.box_total;
+        a.stage_prim = (w.dim == 2 ? 5 : 16) * w.npad;
+    }
     a.mode = h.mode;
     a.Q = h.Q;
     a.x0 = h.x0[0];
